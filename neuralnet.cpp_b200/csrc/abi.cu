@@ -129,6 +129,9 @@ int nnb200_gemm_status(int* host_code)
     int fused = 0;
     NNB_TRY(fused_device_error(&fused));
     if (!*host_code && fused) *host_code = fused | 0x10000000;    // bit 28: norm backward (bulk-copy waits)
+    int f32g = 0;
+    NNB_TRY(f32_gemm_device_error(&f32g));
+    if (!*host_code && f32g) *host_code = f32g | 0x08000000;      // bit 27: fp32 GEMM
     return 0;
 }
 

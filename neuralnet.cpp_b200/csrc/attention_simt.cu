@@ -9,6 +9,7 @@
 // Layout: qkv is (tokens, 3*d) row-major, q | k | v side by side, head h at columns h*dk.. of each;
 // out / dout are (tokens, d); lse and dvec are (B*H*S) with index (b*H + h)*S + i.
 #include "kernels.h"
+#include "simt_tile.cuh"
 
 namespace nnb {
 
@@ -16,62 +17,6 @@ __device__ __forceinline__ float alibi_slope(int h, int H)
 {
     // m_h = 2^(-8h/H), h from 0 (compute_layer.hpp:2179-2187)
     return powf(2.0f, -8.0f * static_cast<float>(h) / static_cast<float>(H));
-}
-
-template <typename T, int DK>
-__global__ void __launch_bounds__(128)
-attn_fwd_simt_kernel(const T* __restrict__ qkv, T* __restrict__ out, float* __restrict__ lse,
-                     const int* __restrict__ doc, int B, int S, int H, int alibi, float scale)
-{
-    __shared__ float qs[4][DK];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long row = static_cast<long long>(blockIdx.x) * 4 + warp;      // (b*H + h)*S + i
-    if (row >= static_cast<long long>(B) * H * S) return;
-    const int i = static_cast<int>(row % S), h = static_cast<int>((row / S) % H), b = static_cast<int>(row / S / H);
-    const int d = H * DK, ld = 3 * d;
-    const T* qp = qkv + (static_cast<size_t>(b) * S + i) * ld + h * DK;
-    for (int c = lane; c < DK; c += 32) qs[warp][c] = to_f32(qp[c]);
-    __syncwarp();
-    const float slope = alibi ? alibi_slope(h, H) : 0.f;
-    const int my_doc = doc ? doc[b * S + i] : 0;
-    const T* kbase = qkv + static_cast<size_t>(b) * S * ld + d + h * DK;
-    const T* vbase = kbase + d;
-    float m = -INFINITY;
-    for (int j = lane; j <= i; j += 32) {
-        if (doc && doc[b * S + j] != my_doc) continue;
-        const T* kp = kbase + static_cast<size_t>(j) * ld;
-        float s = 0.f;
-#pragma unroll 8
-        for (int c = 0; c < DK; ++c) s += qs[warp][c] * to_f32(kp[c]);
-        s = scale * s - slope * static_cast<float>(i - j);
-        m = fmaxf(m, s);
-    }
-    m = warp_max(m);
-    float l = 0.f, o[DK];
-#pragma unroll
-    for (int c = 0; c < DK; ++c) o[c] = 0.f;
-    for (int j = lane; j <= i; j += 32) {
-        if (doc && doc[b * S + j] != my_doc) continue;
-        const T* kp = kbase + static_cast<size_t>(j) * ld;
-        const T* vp = vbase + static_cast<size_t>(j) * ld;
-        float s = 0.f;
-#pragma unroll 8
-        for (int c = 0; c < DK; ++c) s += qs[warp][c] * to_f32(kp[c]);
-        s = scale * s - slope * static_cast<float>(i - j);
-        const float p = expf(s - m);
-        l += p;
-#pragma unroll
-        for (int c = 0; c < DK; ++c) o[c] += p * to_f32(vp[c]);
-    }
-    l = warp_sum(l);
-    const float inv_l = 1.0f / l;
-    T* op = out + (static_cast<size_t>(b) * S + i) * d + h * DK;
-#pragma unroll
-    for (int c = 0; c < DK; ++c) {
-        const float v = warp_sum(o[c]);
-        if (lane == (c & 31)) op[c] = from_f32<T>(v * inv_l);
-    }
-    if (lane == 0) lse[row] = m + logf(l);
 }
 
 // dvec[row] = sum_c dout[i][h*dk+c] * out[i][h*dk+c]  (= R_i = sum_j W_ij P_ij of the reference's
@@ -133,99 +78,241 @@ static int launch_dvec(const T* out, const T* dout, float* dvec, int B, int S, i
     return 0;
 }
 
-// dQ: one warp per query row, lanes over keys
-template <typename T, int DK>
-__global__ void __launch_bounds__(128)
-attn_bwd_dq_simt_kernel(const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
-                        const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc, int B, int S,
-                        int H, int alibi, float scale)
+// ---- tiles of 64 queries x 64 keys; a block of 256 threads per tile row (forward, dQ) or tile column (dK, dV).
+// What bounds them: the fp32 pipe at long sequences; at short ones (few blocks) the chain stage - product - exponential.
+// 8 x 128 x 4 heads of 32, fp32: forward 15 us, dQ 14, dK / dV 18 (with one warp per row and lanes over the keys, whose loads
+// were a row length apart: 123, 132, 179).
+template <int DK> struct SimtDims {
+    static constexpr int KC = DK < 64 ? DK : 64, W = tile_width(DK), ROWS = kTile * (DK + 4);
+};
+
+// score of (i, j) after scale and ALiBi, -inf where the mask leaves nothing
+struct ScoreMask {
+    const int* doc;          // this sequence's document ids, or null
+    int S;
+    float scale, slope;
+    __device__ __forceinline__ bool open(int i, int j) const { return j <= i && i < S && (!doc || doc[j] == doc[i]); }
+    __device__ __forceinline__ float score(float s, int i, int j) const { return scale * s - slope * static_cast<float>(i - j); }
+};
+
+// is anything of the 64 x 64 tile at (i0, j0) open?  Only document masks close tiles on or below the diagonal.
+__device__ __forceinline__ bool tile_open(const ScoreMask& mk, int i0, int j0)
 {
-    __shared__ float qs[4][DK], gs[4][DK];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long row = static_cast<long long>(blockIdx.x) * 4 + warp;
-    if (row >= static_cast<long long>(B) * H * S) return;
-    const int i = static_cast<int>(row % S), h = static_cast<int>((row / S) % H), b = static_cast<int>(row / S / H);
-    const int d = H * DK, ld = 3 * d;
-    const T* qp = qkv + (static_cast<size_t>(b) * S + i) * ld + h * DK;
-    const T* gp = dout + (static_cast<size_t>(b) * S + i) * d + h * DK;
-    for (int c = lane; c < DK; c += 32) { qs[warp][c] = to_f32(qp[c]); gs[warp][c] = to_f32(gp[c]); }
-    __syncwarp();
-    const float slope = alibi ? alibi_slope(h, H) : 0.f;
-    const int my_doc = doc ? doc[b * S + i] : 0;
-    const float L = lse[row], Dv = dvec[row];
-    const T* kbase = qkv + static_cast<size_t>(b) * S * ld + d + h * DK;
-    const T* vbase = kbase + d;
-    float dq[DK];
+    if (!mk.doc) return true;
+    bool any = false;
+    const int i = i0 + (threadIdx.x & 63);
+    for (int u = threadIdx.x >> 6; u < kTile; u += 4) any = any || mk.open(i, j0 + u);
+    return __syncthreads_or(any);
+}
+
+template <typename T, int DK>
+__global__ void __launch_bounds__(256) attn_fwd_simt_kernel(const T* __restrict__ qkv, T* __restrict__ out, float* __restrict__ lse,
+                                                            const int* __restrict__ doc, int B, int S, int H, int alibi, float scale)
+{
+    using D = SimtDims<DK>;
+    extern __shared__ __align__(16) float sm[];
+    float *Qs = sm, *Ks = Qs + DK * kTilePitch, *Vs = Ks + DK * kTilePitch, *Ps = Vs + D::ROWS;
+    const int bh = blockIdx.x % (B * H), qt = static_cast<int>(ceil_div(S, kTile)) - 1 - blockIdx.x / (B * H), h = bh % H, b = bh / H;   // long rows first
+    const int d = H * DK, ld = 3 * d, i0 = qt * kTile, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const T* base = qkv + static_cast<size_t>(b) * S * ld + h * DK;
+    const ScoreMask mk{doc ? doc + static_cast<size_t>(b) * S : nullptr, S, scale, alibi ? alibi_slope(h, H) : 0.f};
+    for (int k = 0; k < DK; k += D::KC) stage_tile<D::KC>(Qs + k * kTilePitch, base, ld, 1, i0, S, k, DK);
+    float m[4], l[4], o[4][D::W];
 #pragma unroll
-    for (int c = 0; c < DK; ++c) dq[c] = 0.f;
-    for (int j = lane; j <= i; j += 32) {
-        if (doc && doc[b * S + j] != my_doc) continue;
-        const T* kp = kbase + static_cast<size_t>(j) * ld;
-        const T* vp = vbase + static_cast<size_t>(j) * ld;
-        float s = 0.f, dp = 0.f;
-#pragma unroll 8
-        for (int c = 0; c < DK; ++c) { s += qs[warp][c] * to_f32(kp[c]); dp += gs[warp][c] * to_f32(vp[c]); }
-        s = scale * s - slope * static_cast<float>(i - j);
-        const float ds = expf(s - L) * (dp - Dv);
+    for (int r = 0; r < 4; ++r) {
+        m[r] = -INFINITY; l[r] = 0.f;
 #pragma unroll
-        for (int c = 0; c < DK; ++c) dq[c] += ds * to_f32(kp[c]);
+        for (int c = 0; c < D::W; ++c) o[r][c] = 0.f;
     }
-    T* dqp = dqkv + (static_cast<size_t>(b) * S + i) * ld + h * DK;
+    for (int j0 = 0; j0 <= i0; j0 += kTile) {
+        if (!tile_open(mk, i0, j0)) continue;
+        __syncthreads();
+        for (int k = 0; k < DK; k += D::KC) stage_tile<D::KC>(Ks + k * kTilePitch, base + d, ld, 1, j0, S, k, DK);
+        stage_rows<DK>(Vs, base + 2 * d, ld, 1, j0, S, 0, DK);
+        __syncthreads();
+        float s[4][4] = {};
+        tile_product<DK>(s, Qs, Ks);
 #pragma unroll
-    for (int c = 0; c < DK; ++c) {
-        const float v = warp_sum(dq[c]);
-        if (lane == (c & 31)) dqp[c] = from_f32<T>(scale * v);
+        for (int r = 0; r < 4; ++r) {
+            const int i = i0 + ty * 4 + r;
+            float mx = m[r];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int j = j0 + tx * 4 + c;
+                s[r][c] = mk.open(i, j) ? mk.score(s[r][c], i, j) : -INFINITY;
+                mx = fmaxf(mx, s[r][c]);
+            }
+            mx = row_max16(mx);
+            const float ref = mx == -INFINITY ? 0.f : mx, back = expf(m[r] - ref);
+            float sum = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) { s[r][c] = expf(s[r][c] - ref); sum += s[r][c]; }
+            l[r] = l[r] * back + row_sum16(sum);
+            m[r] = mx;
+#pragma unroll
+            for (int c = 0; c < D::W; ++c) o[r][c] *= back;
+        }
+        put_transposed(Ps, s);
+        __syncthreads();
+        tile_rows_product<D::W, DK>(o, Ps, Vs);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int i = i0 + ty * 4 + r;
+        if (i >= S) continue;
+        const float inv = 1.0f / l[r];
+        T* op = out + (static_cast<size_t>(b) * S + i) * d + h * DK;
+#pragma unroll
+        for (int c = 0; c < D::W; ++c)
+            if (tile_col<D::W>(c) < DK) op[tile_col<D::W>(c)] = from_f32<T>(o[r][c] * inv);
+        if (tx == 0) lse[(static_cast<size_t>(b) * H + h) * S + i] = m[r] + logf(l[r]);
     }
 }
 
-// dK, dV: one warp per key row, lanes over the queries that see it
+// dQ_i = scale sum_j P_ij (dP_ij - D_i) k_j
 template <typename T, int DK>
-__global__ void __launch_bounds__(128)
-attn_bwd_dkv_simt_kernel(const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
-                         const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc, int B, int S,
-                         int H, int alibi, float scale)
+__global__ void __launch_bounds__(256) attn_bwd_dq_simt_kernel(const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
+                                                               const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc,
+                                                               int B, int S, int H, int alibi, float scale)
 {
-    __shared__ float ks[4][DK], vs[4][DK];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long row = static_cast<long long>(blockIdx.x) * 4 + warp;
-    if (row >= static_cast<long long>(B) * H * S) return;
-    const int j = static_cast<int>(row % S), h = static_cast<int>((row / S) % H), b = static_cast<int>(row / S / H);
-    const int d = H * DK, ld = 3 * d;
-    const T* kp = qkv + (static_cast<size_t>(b) * S + j) * ld + d + h * DK;
-    for (int c = lane; c < DK; c += 32) { ks[warp][c] = to_f32(kp[c]); vs[warp][c] = to_f32(kp[d + c]); }
-    __syncwarp();
-    const float slope = alibi ? alibi_slope(h, H) : 0.f;
-    const int my_doc = doc ? doc[b * S + j] : 0;
-    const long long row0 = (static_cast<long long>(b) * H + h) * S;
-    float dk[DK], dv[DK];
-#pragma unroll
-    for (int c = 0; c < DK; ++c) { dk[c] = 0.f; dv[c] = 0.f; }
-    for (int i = j + lane; i < S; i += 32) {
-        if (doc && doc[b * S + i] != my_doc) continue;
-        const T* qp = qkv + (static_cast<size_t>(b) * S + i) * ld + h * DK;
-        const T* gp = dout + (static_cast<size_t>(b) * S + i) * d + h * DK;
-        float s = 0.f, dp = 0.f;
-#pragma unroll 8
-        for (int c = 0; c < DK; ++c) { s += to_f32(qp[c]) * ks[warp][c]; dp += to_f32(gp[c]) * vs[warp][c]; }
-        s = scale * s - slope * static_cast<float>(i - j);
-        const float p = expf(s - lse[row0 + i]);
-        const float ds = p * (dp - dvec[row0 + i]);
-#pragma unroll
-        for (int c = 0; c < DK; ++c) { dk[c] += ds * to_f32(qp[c]); dv[c] += p * to_f32(gp[c]); }
+    using D = SimtDims<DK>;
+    extern __shared__ __align__(16) float sm[];
+    float *Qs = sm, *Gs = Qs + DK * kTilePitch, *Ks = Gs + DK * kTilePitch, *Vs = Ks + D::KC * kTilePitch, *Kr = Vs + D::KC * kTilePitch, *Ps = Kr + D::ROWS;
+    const int bh = blockIdx.x % (B * H), qt = static_cast<int>(ceil_div(S, kTile)) - 1 - blockIdx.x / (B * H), h = bh % H, b = bh / H;
+    const int d = H * DK, ld = 3 * d, i0 = qt * kTile, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const T* base = qkv + static_cast<size_t>(b) * S * ld + h * DK;
+    const T* gbase = dout + static_cast<size_t>(b) * S * d + h * DK;
+    const ScoreMask mk{doc ? doc + static_cast<size_t>(b) * S : nullptr, S, scale, alibi ? alibi_slope(h, H) : 0.f};
+    const size_t row0 = (static_cast<size_t>(b) * H + h) * S;
+    for (int k = 0; k < DK; k += D::KC) {
+        stage_tile<D::KC>(Qs + k * kTilePitch, base, ld, 1, i0, S, k, DK);
+        stage_tile<D::KC>(Gs + k * kTilePitch, gbase, d, 1, i0, S, k, DK);
     }
-    T* dkp = dqkv + (static_cast<size_t>(b) * S + j) * ld + d + h * DK;
+    float L[4], Dv[4], dq[4][D::W];
 #pragma unroll
-    for (int c = 0; c < DK; ++c) {
-        const float a = warp_sum(dk[c]), bsum = warp_sum(dv[c]);
-        if (lane == (c & 31)) { dkp[c] = from_f32<T>(scale * a); dkp[d + c] = from_f32<T>(bsum); }
+    for (int r = 0; r < 4; ++r) {
+        const int i = i0 + ty * 4 + r;
+        L[r] = i < S ? lse[row0 + i] : 0.f;
+        Dv[r] = i < S ? dvec[row0 + i] : 0.f;
+#pragma unroll
+        for (int c = 0; c < D::W; ++c) dq[r][c] = 0.f;
+    }
+    for (int j0 = 0; j0 <= i0; j0 += kTile) {
+        if (!tile_open(mk, i0, j0)) continue;
+        float s[4][4] = {}, dp[4][4] = {};
+        for (int k = 0; k < DK; k += D::KC) {
+            __syncthreads();
+            stage_tile<D::KC>(Ks, base + d, ld, 1, j0, S, k, DK);
+            stage_tile<D::KC>(Vs, base + 2 * d, ld, 1, j0, S, k, DK);
+            if (k == 0) stage_rows<DK>(Kr, base + d, ld, 1, j0, S, 0, DK);
+            __syncthreads();
+            tile_product<D::KC>(s, Qs + k * kTilePitch, Ks);
+            tile_product<D::KC>(dp, Gs + k * kTilePitch, Vs);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int i = i0 + ty * 4 + r;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int j = j0 + tx * 4 + c;
+                s[r][c] = mk.open(i, j) ? expf(mk.score(s[r][c], i, j) - L[r]) * (dp[r][c] - Dv[r]) : 0.f;
+            }
+        }
+        put_transposed(Ps, s);
+        __syncthreads();
+        tile_rows_product<D::W, DK>(dq, Ps, Kr);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int i = i0 + ty * 4 + r;
+        if (i >= S) continue;
+        T* p = dqkv + (static_cast<size_t>(b) * S + i) * ld + h * DK;
+#pragma unroll
+        for (int c = 0; c < D::W; ++c)
+            if (tile_col<D::W>(c) < DK) p[tile_col<D::W>(c)] = from_f32<T>(scale * dq[r][c]);
     }
 }
+
+// dK_j = scale sum_i P_ij (dP_ij - D_i) q_i ; dV_j = sum_i P_ij dO_i.  Rows of the tile are keys, columns queries.
+template <typename T, int DK>
+__global__ void __launch_bounds__(256) attn_bwd_dkv_simt_kernel(const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
+                                                                const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc,
+                                                                int B, int S, int H, int alibi, float scale)
+{
+    using D = SimtDims<DK>;
+    extern __shared__ __align__(16) float sm[];
+    float *Ks = sm, *Vs = Ks + D::KC * kTilePitch, *Qs = Vs + D::KC * kTilePitch, *Gs = Qs + D::KC * kTilePitch, *Qr = Gs + D::KC * kTilePitch,
+          *Gr = Qr + D::ROWS, *Ps = Gr + D::ROWS, *Ss = Ps + kTileFloats;
+    const int bh = blockIdx.x % (B * H), kt = blockIdx.x / (B * H), h = bh % H, b = bh / H;      // the first keys are seen by the most queries
+    const int d = H * DK, ld = 3 * d, j0 = kt * kTile, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const T* base = qkv + static_cast<size_t>(b) * S * ld + h * DK;
+    const T* gbase = dout + static_cast<size_t>(b) * S * d + h * DK;
+    const ScoreMask mk{doc ? doc + static_cast<size_t>(b) * S : nullptr, S, scale, alibi ? alibi_slope(h, H) : 0.f};
+    const size_t row0 = (static_cast<size_t>(b) * H + h) * S;
+    float dk[4][D::W], dv[4][D::W];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < D::W; ++c) { dk[r][c] = 0.f; dv[r][c] = 0.f; }
+    for (int i0 = j0; i0 < S; i0 += kTile) {
+        if (!tile_open(mk, i0, j0)) continue;
+        float s[4][4] = {}, dp[4][4] = {};
+        for (int k = 0; k < DK; k += D::KC) {
+            __syncthreads();
+            if (DK > D::KC || i0 == j0) {                        // one chunk: the keys stay (the diagonal tile is always open)
+                stage_tile<D::KC>(Ks, base + d, ld, 1, j0, S, k, DK);
+                stage_tile<D::KC>(Vs, base + 2 * d, ld, 1, j0, S, k, DK);
+            }
+            stage_tile<D::KC>(Qs, base, ld, 1, i0, S, k, DK);
+            stage_tile<D::KC>(Gs, gbase, d, 1, i0, S, k, DK);
+            if (k == 0) { stage_rows<DK>(Qr, base, ld, 1, i0, S, 0, DK); stage_rows<DK>(Gr, gbase, d, 1, i0, S, 0, DK); }
+            __syncthreads();
+            tile_product<D::KC>(s, Ks, Qs);
+            tile_product<D::KC>(dp, Vs, Gs);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int i = i0 + tx * 4 + c;
+            const float L = i < S ? lse[row0 + i] : 0.f, Dv = i < S ? dvec[row0 + i] : 0.f;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int j = j0 + ty * 4 + r;
+                const float p = mk.open(i, j) ? expf(mk.score(s[r][c], i, j) - L) : 0.f;
+                s[r][c] = p;
+                dp[r][c] = p * (dp[r][c] - Dv);
+            }
+        }
+        put_transposed(Ps, s);
+        put_transposed(Ss, dp);
+        __syncthreads();
+        tile_rows_product<D::W, DK>(dv, Ps, Gr);
+        tile_rows_product<D::W, DK>(dk, Ss, Qr);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int j = j0 + ty * 4 + r;
+        if (j >= S) continue;
+        T* p = dqkv + (static_cast<size_t>(b) * S + j) * ld + d + h * DK;
+#pragma unroll
+        for (int c = 0; c < D::W; ++c) {
+            const int col = tile_col<D::W>(c);
+            if (col < DK) { p[col] = from_f32<T>(scale * dk[r][c]); p[d + col] = from_f32<T>(dv[r][c]); }
+        }
+    }
+}
+
+template <int DK> constexpr int simt_smem_fwd() { return (2 * DK * kTilePitch + SimtDims<DK>::ROWS + kTileFloats) * 4; }
+template <int DK> constexpr int simt_smem_dq() { return (2 * DK * kTilePitch + 2 * SimtDims<DK>::KC * kTilePitch + SimtDims<DK>::ROWS + kTileFloats) * 4; }
+template <int DK> constexpr int simt_smem_dkv() { return (4 * SimtDims<DK>::KC * kTilePitch + 2 * SimtDims<DK>::ROWS + 2 * kTileFloats) * 4; }
+static_assert(simt_smem_dq<128>() <= 232448 && simt_smem_dkv<128>() <= 232448, "exceeds the 227 KB of shared memory a block may use");
 
 template <typename T, int DK>
 static int fwd_dk(const T* qkv, T* out, float* lse, const int* doc, int B, int S, int H, int alibi, cudaStream_t s)
 {
-    const long long rows = static_cast<long long>(B) * H * S;
-    attn_fwd_simt_kernel<T, DK><<<static_cast<unsigned>(ceil_div(rows, 4)), 128, 0, s>>>(
+    NNB_ARG_CHECK(ceil_div(S, kTile) * B * H <= INT_MAX, "too many tiles for one launch");
+    static PerDeviceOnce once;
+    NNB_TRY(once.run([] { return cudaFuncSetAttribute(attn_fwd_simt_kernel<T, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, simt_smem_fwd<DK>()); }));
+    attn_fwd_simt_kernel<T, DK><<<static_cast<unsigned>(ceil_div(S, kTile) * B * H), 256, simt_smem_fwd<DK>(), s>>>(
         qkv, out, lse, doc, B, S, H, alibi, 1.0f / sqrtf(static_cast<float>(DK)));
     NNB_LAUNCH_CHECK();
     return 0;
@@ -234,13 +321,18 @@ template <typename T, int DK>
 static int bwd_dk(const T* qkv, const T* out, const T* dout, const float* lse, float* dvec, T* dqkv, const int* doc,
                   int B, int S, int H, int alibi, cudaStream_t s)
 {
-    const long long rows = static_cast<long long>(B) * H * S;
+    NNB_ARG_CHECK(ceil_div(S, kTile) * B * H <= INT_MAX, "too many tiles for one launch");
+    static PerDeviceOnce once;
+    NNB_TRY(once.run([] {
+        const cudaError_t e = cudaFuncSetAttribute(attn_bwd_dq_simt_kernel<T, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, simt_smem_dq<DK>());
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(attn_bwd_dkv_simt_kernel<T, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, simt_smem_dkv<DK>());
+    }));
     const float scale = 1.0f / sqrtf(static_cast<float>(DK));
     NNB_TRY(launch_dvec<T>(out, dout, dvec, B, S, H, DK, s));
-    const unsigned grid = static_cast<unsigned>(ceil_div(rows, 4));
-    attn_bwd_dq_simt_kernel<T, DK><<<grid, 128, 0, s>>>(qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale);
+    const unsigned grid = static_cast<unsigned>(ceil_div(S, kTile) * B * H);
+    attn_bwd_dq_simt_kernel<T, DK><<<grid, 256, simt_smem_dq<DK>(), s>>>(qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale);
     NNB_LAUNCH_CHECK();
-    attn_bwd_dkv_simt_kernel<T, DK><<<grid, 128, 0, s>>>(qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale);
+    attn_bwd_dkv_simt_kernel<T, DK><<<grid, 256, simt_smem_dkv<DK>(), s>>>(qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale);
     NNB_LAUNCH_CHECK();
     return 0;
 }

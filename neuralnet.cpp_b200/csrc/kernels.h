@@ -13,11 +13,16 @@ struct DecodeLayer { long long wqkv, bqkv, wo, bo, g1, be1, w1, b1, w2, b2, g2, 
 struct DecodeLayout { long long tok_emb, pos_emb, lnf_g, lnf_b, lm_w, lm_b; std::vector<DecodeLayer> layers; };
 DecodeLayout decode_layout(const ::nnb200_gpt_config& c);
 
-// ---- gemm_simt.cu : fp32, arbitrary strides, optional batch
+// ---- gemm_f32.cu : fp32 products on the bf16 tensor cores; each operand contiguous along one index, optional batch
 int sgemm_strided(const float* A, const float* B, float* C, int M, int N, int K, long long sam, long long sak,
                   long long sbn, long long sbk, long long ldc, int batch, long long batch_a, long long batch_b,
                   long long batch_c, float alpha, const float* bias_n, const float* bias_m, const float* residual,
                   int accumulate, cudaStream_t stream);
+
+// fp32 rows times bf16 rows: C[M, N] = A[M, K] B[N, K]^T (+ bias_n) (+ residual), C fp32
+int gemm_f32_bf16(const float* A, const bf16* B, float* C, int M, int N, int K, const float* bias_n, const float* residual,
+                  cudaStream_t stream);
+int f32_gemm_device_error(int* code);      // reads and clears
 
 // ---- gemm_tcgen05.cu : bf16 operands, fp32 accumulate in TMEM
 int gemm_bf16(const bf16* A, const bf16* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
