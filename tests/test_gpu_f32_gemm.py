@@ -1,0 +1,89 @@
+"""fp32 GEMM on the bf16 tensor cores (nnb200_gemm_f32) at the edges of its tiles and splits, against float64."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def g():
+    from tests import gpu_util
+    return gpu_util
+
+
+# one element; one tile and one past it (128 rows, 64 or 128 columns, 64 of K); K that splits over 2, 4 and 8 CTAs of a
+# cluster, with a last rank that has nothing; rows no 16-byte load can take; several tiles per persistent CTA
+SHAPES = [(1, 1, 1), (128, 64, 64), (129, 65, 65), (128, 128, 192), (100, 60, 1000), (384, 128, 1024), (70, 40, 577), (805, 377, 697),
+          (3000, 2600, 200)]
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", SHAPES)
+def test_gemm_f32_against_float64(g, M, N, K, a_mn, b_mn):
+    r = np.random.default_rng(M + N + K)
+    A, B = r.standard_normal((M, K)).astype(np.float32), r.standard_normal((N, K)).astype(np.float32)
+    c0, bias = r.standard_normal((M, N)).astype(np.float32), r.standard_normal(N).astype(np.float32)
+    a, b, bv = g.dev(A.T if a_mn else A), g.dev(B.T if b_mn else B), g.dev(bias)
+    scale = np.abs(A.astype(np.float64)) @ np.abs(B.astype(np.float64)).T
+    for accumulate in (0, 1):
+        c = g.dev(c0)
+        g.call("nnb200_gemm_f32", g.ptr(a), g.ptr(b), g.ptr(c), M, N, K, M if a_mn else K, N if b_mn else K, N, a_mn, b_mn, C.c_float(0.5),
+               g.ptr(bv), None, accumulate, g.stream())
+        want = 0.5 * A.astype(np.float64) @ B.astype(np.float64).T + bias + (c0 if accumulate else 0)
+        # dropped products below 2^-24 of |a||b|; at most six steps of the tensor core's sum at full size per 64 of K, each
+        # off by 2^-23; one rounding per 64 of K and per split, and three in the epilogue
+        bound = 0.5 * scale * (2.0 ** -24 + 6 * 2.0 ** -23 + (K / 64 + 8) * 2.0 ** -24) + 3 * 2.0 ** -23 * (np.abs(want) + np.abs(c0) + 1)
+        assert (np.abs(g.host(c) - want) <= bound).all()
+    assert g.gemm_status() == 0
+
+
+def test_gemm_f32_non_finite_and_huge_operands(g):
+    """What an infinity, a NaN or a value that bf16 rounds to infinity makes of a result is what fp32 arithmetic makes of it."""
+    r = np.random.default_rng(3)
+    A, B = r.standard_normal((300, 200)).astype(np.float32), r.standard_normal((150, 200)).astype(np.float32)
+    A[5, 3], A[9, 2], B[4, 9], A[7, 1], B[3, 1] = np.inf, np.nan, -np.inf, 3.3e38, 0.0
+    a, b, c = g.dev(A), g.dev(B), g.dev(np.zeros((300, 150), np.float32))
+    g.call("nnb200_gemm_f32", g.ptr(a), g.ptr(b), g.ptr(c), 300, 150, 200, 200, 200, 150, 0, 0, C.c_float(1.0), None, None, 0, g.stream())
+    with np.errstate(all="ignore"):
+        want = A.astype(np.float64) @ B.astype(np.float64).T
+        want = np.where(np.abs(want) > np.finfo(np.float32).max, np.sign(want) * np.inf, want)
+    got = g.host(c)
+    rows, cols = np.delete(np.arange(300), 7), np.arange(150)          # row 7 overflows in part: order-dependent, except at B = 0
+    assert np.array_equal(np.isnan(got[rows]), np.isnan(want[rows])) and np.array_equal(np.isposinf(got[rows]), np.isposinf(want[rows]))
+    fine = np.isfinite(want[rows])
+    assert np.abs(got[rows][fine] - want[rows][fine]).max() < 1e-3
+    assert abs(got[7, 3] - want[7, 3]) < 1e-3
+
+
+@pytest.mark.parametrize("dk", [8, 32, 64, 128])
+@pytest.mark.parametrize("S", [1, 63, 64, 65, 200])
+@pytest.mark.parametrize("docs", [False, True])
+def test_attention_f32_tile_edges(g, dk, S, docs):
+    """Sequence lengths around the 64-row tiles of the fp32 attention kernels, with documents that close whole tiles: against
+    float64 autograd."""
+    import torch
+    B, H = 2, 3
+    d = H * dk
+    gen = torch.Generator(device="cuda").manual_seed(S + dk)
+    qkv = torch.randn(B * S, 3 * d, device="cuda", generator=gen)
+    dout = torch.randn(B * S, d, device="cuda", generator=gen)
+    doc = (torch.arange(B * S, device="cuda", dtype=torch.int32) // 50).contiguous() if docs else None
+    out, lse, dqkv, dvec = torch.empty_like(dout), torch.empty(B * H * S, device="cuda"), torch.empty_like(qkv), torch.empty(B * H * S, device="cuda")
+    g.call("nnb200_attention_forward", g.ptr(qkv), g.ptr(out), g.ptr(lse), g.ptr(doc), None, B, S, H, dk, 1, 0, g.stream())
+    g.call("nnb200_attention_backward", g.ptr(qkv), g.ptr(out), g.ptr(dout), g.ptr(lse), g.ptr(dvec), g.ptr(dqkv), g.ptr(doc), None, B, S, H, dk, 1, 0,
+           g.stream())
+    x = qkv.double().requires_grad_()
+    q, k, v = x.view(B, S, 3, H, dk).permute(2, 0, 3, 1, 4)
+    i = torch.arange(S, device="cuda")
+    slope = torch.exp2(-8.0 * torch.arange(H, device="cuda", dtype=torch.float64) / H)
+    s = q @ k.transpose(-1, -2) / dk ** 0.5 - slope[None, :, None, None] * (i[:, None] - i[None, :])
+    mask = (i[None, :] <= i[:, None])[None, None]
+    if docs:
+        mask = mask & (doc.view(B, 1, S, 1) == doc.view(B, 1, 1, S))
+    ref = (s.masked_fill(~mask, float("-inf")).softmax(-1) @ v).transpose(1, 2).reshape(B * S, d)
+    ref.backward(dout.double())
+    # fp32 sums of up to 200 terms and an exponential of arguments up to about 50 (error 50 x 2^-24): 1e-5 of the norm
+    assert (out - ref).norm() <= 1e-5 * ref.norm()
+    assert (dqkv - x.grad).norm() <= 1e-5 * x.grad.norm()
