@@ -105,18 +105,24 @@ __device__ __forceinline__ bool tile_open(const ScoreMask& mk, int i0, int j0)
     return __syncthreads_or(any);
 }
 
+// Queries are rows q0 .. S - 1 of a sequence of S keys (q0 = 0 in training; a prompt pass continues behind q0 cached rows), so
+// q and out point at the row of query q0; `lse` may be null.
 template <typename T, int DK>
-__global__ void __launch_bounds__(256) attn_fwd_simt_kernel(const T* __restrict__ qkv, T* __restrict__ out, float* __restrict__ lse,
-                                                            const int* __restrict__ doc, int B, int S, int H, int alibi, float scale)
+__global__ void __launch_bounds__(256) attn_fwd_simt_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ kc, const T* __restrict__ vc,
+                                                            long long ldk, T* __restrict__ out, float* __restrict__ lse, const int* __restrict__ doc,
+                                                            int B, int S, int q0, int H, int alibi, float scale)
 {
     using D = SimtDims<DK>;
     extern __shared__ __align__(16) float sm[];
     float *Qs = sm, *Ks = Qs + DK * kTilePitch, *Vs = Ks + DK * kTilePitch, *Ps = Vs + D::ROWS;
-    const int bh = blockIdx.x % (B * H), qt = static_cast<int>(ceil_div(S, kTile)) - 1 - blockIdx.x / (B * H), h = bh % H, b = bh / H;   // long rows first
-    const int d = H * DK, ld = 3 * d, i0 = qt * kTile, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const T* base = qkv + static_cast<size_t>(b) * S * ld + h * DK;
+    const int nq = S - q0;
+    const int bh = blockIdx.x % (B * H), qt = static_cast<int>(ceil_div(nq, kTile)) - 1 - blockIdx.x / (B * H), h = bh % H, b = bh / H;   // long rows first
+    const int d = H * DK, i0 = q0 + qt * kTile, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const T* qb = q + static_cast<size_t>(b) * nq * ldq + h * DK;
+    const T* kb = kc + static_cast<size_t>(b) * S * ldk + h * DK;
+    const T* vb = vc + static_cast<size_t>(b) * S * ldk + h * DK;
     const ScoreMask mk{doc ? doc + static_cast<size_t>(b) * S : nullptr, S, scale, alibi ? alibi_slope(h, H) : 0.f};
-    for (int k = 0; k < DK; k += D::KC) stage_tile<D::KC>(Qs + k * kTilePitch, base, ld, 1, i0, S, k, DK);
+    for (int k = 0; k < DK; k += D::KC) stage_tile<D::KC>(Qs + k * kTilePitch, qb, ldq, 1, i0 - q0, nq, k, DK);
     float m[4], l[4], o[4][D::W];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -124,11 +130,11 @@ __global__ void __launch_bounds__(256) attn_fwd_simt_kernel(const T* __restrict_
 #pragma unroll
         for (int c = 0; c < D::W; ++c) o[r][c] = 0.f;
     }
-    for (int j0 = 0; j0 <= i0; j0 += kTile) {
+    for (int j0 = 0; j0 < S && j0 < i0 + kTile; j0 += kTile) {
         if (!tile_open(mk, i0, j0)) continue;
         __syncthreads();
-        for (int k = 0; k < DK; k += D::KC) stage_tile<D::KC>(Ks + k * kTilePitch, base + d, ld, 1, j0, S, k, DK);
-        stage_rows<DK>(Vs, base + 2 * d, ld, 1, j0, S, 0, DK);
+        for (int k = 0; k < DK; k += D::KC) stage_tile<D::KC>(Ks + k * kTilePitch, kb, ldk, 1, j0, S, k, DK);
+        stage_rows<DK>(Vs, vb, ldk, 1, j0, S, 0, DK);
         __syncthreads();
         float s[4][4] = {};
         tile_product<DK>(s, Qs, Ks);
@@ -161,11 +167,11 @@ __global__ void __launch_bounds__(256) attn_fwd_simt_kernel(const T* __restrict_
         const int i = i0 + ty * 4 + r;
         if (i >= S) continue;
         const float inv = 1.0f / l[r];
-        T* op = out + (static_cast<size_t>(b) * S + i) * d + h * DK;
+        T* op = out + (static_cast<size_t>(b) * nq + i - q0) * d + h * DK;
 #pragma unroll
         for (int c = 0; c < D::W; ++c)
             if (tile_col<D::W>(c) < DK) op[tile_col<D::W>(c)] = from_f32<T>(o[r][c] * inv);
-        if (tx == 0) lse[(static_cast<size_t>(b) * H + h) * S + i] = m[r] + logf(l[r]);
+        if (tx == 0 && lse) lse[(static_cast<size_t>(b) * H + h) * S + i] = m[r] + logf(l[r]);
     }
 }
 
@@ -307,13 +313,14 @@ template <int DK> constexpr int simt_smem_dkv() { return (4 * SimtDims<DK>::KC *
 static_assert(simt_smem_dq<128>() <= 232448 && simt_smem_dkv<128>() <= 232448, "exceeds the 227 KB of shared memory a block may use");
 
 template <typename T, int DK>
-static int fwd_dk(const T* qkv, T* out, float* lse, const int* doc, int B, int S, int H, int alibi, cudaStream_t s)
+static int fwd_dk(const T* q, long long ldq, const T* k, const T* v, long long ldk, T* out, float* lse, const int* doc, int B, int S, int q0,
+                  int H, int alibi, cudaStream_t s)
 {
-    NNB_ARG_CHECK(ceil_div(S, kTile) * B * H <= INT_MAX, "too many tiles for one launch");
+    NNB_ARG_CHECK(ceil_div(S - q0, kTile) * B * H <= INT_MAX, "too many tiles for one launch");
     static PerDeviceOnce once;
     NNB_TRY(once.run([] { return cudaFuncSetAttribute(attn_fwd_simt_kernel<T, DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, simt_smem_fwd<DK>()); }));
-    attn_fwd_simt_kernel<T, DK><<<static_cast<unsigned>(ceil_div(S, kTile) * B * H), 256, simt_smem_fwd<DK>(), s>>>(
-        qkv, out, lse, doc, B, S, H, alibi, 1.0f / sqrtf(static_cast<float>(DK)));
+    attn_fwd_simt_kernel<T, DK><<<static_cast<unsigned>(ceil_div(S - q0, kTile) * B * H), 256, simt_smem_fwd<DK>(), s>>>(
+        q, ldq, k, v, ldk, out, lse, doc, B, S, q0, H, alibi, 1.0f / sqrtf(static_cast<float>(DK)));
     NNB_LAUNCH_CHECK();
     return 0;
 }
@@ -352,7 +359,16 @@ int attention_fwd_simt(const T* qkv, T* out, float* lse, const int* doc, int B, 
                        cudaStream_t s)
 {
     if (static_cast<long long>(B) * S * H == 0) return 0;
-    DISPATCH_DK(dk, (fwd_dk<T, DKC>(qkv, out, lse, doc, B, S, H, alibi, s)));
+    const int d = H * dk;
+    DISPATCH_DK(dk, (fwd_dk<T, DKC>(qkv, 3 * d, qkv + d, qkv + 2 * d, 3 * d, out, lse, doc, B, S, 0, H, alibi, s)));
+}
+
+bool attention_prompt_supported(int dk) { return dk == 8 || dk == 16 || dk == 32 || dk == 64 || dk == 128; }
+int attention_prompt(const float* qkv, const float* k_cache, const float* v_cache, float* out, int start, int n, int H, int dk, int alibi, cudaStream_t s)
+{
+    if (n == 0) return 0;
+    const int d = H * dk;
+    DISPATCH_DK(dk, (fwd_dk<float, DKC>(qkv, 3 * d, k_cache, v_cache, d, out, nullptr, nullptr, 1, start + n, start, H, alibi, s)));
 }
 template <typename T>
 int attention_bwd_simt(const T* qkv, const T* out, const T* dout, const float* lse, float* dvec, T* dqkv,

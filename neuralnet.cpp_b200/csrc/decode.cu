@@ -10,6 +10,7 @@
 // few KB), the attention over the cache is split over chunks of 32 cached rows per head, and the token id, position
 // and cache length are read from device memory, so that the launches of a token are the same every time and a caller
 // may replay them as a CUDA graph (nnb200_gpt_forward_step_dev).
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -18,7 +19,13 @@
 
 namespace nnb {
 
-struct DecodeWs { size_t kv, table, x, xn, qkv, att, xmid, h1, h2, logits, step, part, count, total; };
+struct DecodeWs { size_t kv, table, x, xn, qkv, att, xmid, h1, h2, logits, step, part, count, total;
+                  size_t p_tok, p_x, p_xn, p_qkv, p_att, p_mid, p_h1, p_h2, p_stat; };
+// Rows of a prompt that one pass takes (longer prompts go in several): enough to fill the GEMM's tiles, 60 MB of
+// activations for a model of width 1024.
+constexpr int kPromptRows = 1024;
+// Shorter prompts go through the single-token kernels: a pass costs about as much as several tokens whatever its length.
+constexpr int kPromptMin = 8;
 constexpr int kDecodeChunk = 32;                    // cached rows per attention block: a block is one round of loads, bound by their latency
 static DecodeWs decode_ws(const nnb200_gpt_config& c)
 {
@@ -34,6 +41,9 @@ static DecodeWs decode_ws(const nnb200_gpt_config& c)
     W.step = take(4);                                            // token id, position, cache length
     W.part = take(static_cast<size_t>(c.heads) * chunks * (d / c.heads + 2));   // per (head, chunk): maximum, sum, weighted values
     W.count = take(static_cast<size_t>(c.heads));               // chunks of a head that have finished (back to zero after each step)
+    const size_t R = std::min<size_t>(S, kPromptRows);
+    W.p_tok = take(R); W.p_x = take(R * d); W.p_xn = take(R * d); W.p_qkv = take(R * 3 * d); W.p_att = take(R * d); W.p_mid = take(R * d);
+    W.p_h1 = take(R * fc1); W.p_h2 = take(R * c.d_ff); W.p_stat = take(2 * R);
     W.total = off;
     return W;
 }
@@ -258,6 +268,81 @@ static int forward_step_t(const nnb200_gpt_config& c, const float* P, const WT* 
     return gemv<WT, 1>(Wt + L.lm_w, x, P + L.lnf_g, PB(L.lnf_b), ln, P + L.lm_b, nullptr, logits_out ? logits_out : F(W.logits), c.vocab, d, s);
 }
 
+// Y[n, out] = X[n, in] W[out, in]^T + bias (+ residual), fp32 rows times fp32 or bf16 weights
+static int prompt_linear(const float* X, const float* W, const float* bias, const float* residual, float* Y, int n, int in, int out, cudaStream_t s)
+{
+    return sgemm_strided(X, W, Y, n, out, in, in, 1, in, 1, out, 1, 0, 0, 0, 1.0f, bias, nullptr, residual, 0, s);
+}
+static int prompt_linear(const float* X, const bf16* W, const float* bias, const float* residual, float* Y, int n, int in, int out, cudaStream_t s)
+{
+    return gemm_f32_bf16(X, W, Y, n, out, in, bias, residual, s);
+}
+
+// n <= kPromptRows prompt tokens (device) at cache rows start ..: the layers as products over all rows, with the fp32
+// activations, weights and cache of the single-token kernels.  Leaves the last layer's output rows in p_x.
+// A token at a time reads every weight per token: 501 tokens of the 12-layer benchmark model took 260 ms.
+template <typename WT>
+static int prompt_pass_t(const nnb200_gpt_config& c, const float* P, const WT* Wt, uint8_t* ws, const int* tokens, int start, int n, cudaStream_t s)
+{
+    const DecodeLayout L = decode_layout(c);
+    const DecodeWs W = decode_ws(c);
+    const int d = c.d_model, ff = c.d_ff, fc1 = c.act == 1 ? 2 * ff : ff, dk = d / c.heads;
+    const bool ln = c.norm == 0;
+    auto F = [&](size_t off) { return reinterpret_cast<float*>(ws + off); };
+    auto PB = [&](long long off) { return off >= 0 ? P + off : nullptr; };
+    const float* pos_table = c.pos == 0 ? P + L.pos_emb : (c.pos == 1 ? F(W.table) : nullptr);
+    float *x = F(W.p_x), *xn = F(W.p_xn), *qkv = F(W.p_qkv), *att = F(W.p_att), *mid = F(W.p_mid), *h1 = F(W.p_h1), *h2 = F(W.p_h2);
+    float *rinv = F(W.p_stat), *mean = rinv + n;
+    // rows of the tables and of the cache begin at `start`; the kernels count from there (n <= seq - start)
+    NNB_TRY(embed_fwd<float>(P + L.tok_emb, pos_table ? pos_table + static_cast<size_t>(start) * d : nullptr, tokens, x, n, c.seq, d, c.vocab, s));
+    const size_t layer_kv = static_cast<size_t>(2) * c.seq * d;
+    for (int l = 0; l < c.layers; ++l) {
+        const DecodeLayer& lp = L.layers[l];
+        float* kc = F(W.kv) + static_cast<size_t>(l) * layer_kv;
+        float* vc = kc + static_cast<size_t>(c.seq) * d;
+        NNB_TRY(norm_fwd<float>(x, P + lp.g1, PB(lp.be1), xn, rinv, mean, n, d, ln, s));
+        NNB_TRY(prompt_linear(xn, Wt + lp.wqkv, P + lp.bqkv, nullptr, qkv, n, d, 3 * d, s));
+        if (c.pos == 3) NNB_TRY(rope_apply<float>(qkv, F(W.table) + static_cast<size_t>(start) * (dk / 2), n, c.seq, c.heads, dk, 3 * d, false, s));
+        for (int w = 0; w < 2; ++w)
+            NNB_CUDA_CHECK(cudaMemcpy2DAsync((w ? vc : kc) + static_cast<size_t>(start) * d, static_cast<size_t>(d) * 4, qkv + (1 + w) * d,
+                                             static_cast<size_t>(3) * d * 4, static_cast<size_t>(d) * 4, n, cudaMemcpyDeviceToDevice, s));
+        NNB_TRY(attention_prompt(qkv, kc, vc, att, start, n, c.heads, dk, c.pos == 2 ? 1 : 0, s));
+        NNB_TRY(prompt_linear(att, Wt + lp.wo, P + lp.bo, x, mid, n, d, d, s));
+        NNB_TRY(norm_fwd<float>(mid, P + lp.g2, PB(lp.be2), xn, rinv, mean, n, d, ln, s));
+        NNB_TRY(prompt_linear(xn, Wt + lp.w1, P + lp.b1, nullptr, h1, n, d, fc1, s));
+        NNB_TRY(act_fwd<float>(h1, h2, n, ff, c.act == 1, s));
+        NNB_TRY(prompt_linear(h2, Wt + lp.w2, P + lp.b2, mid, x, n, ff, d, s));
+    }
+    return 0;
+}
+
+template <typename WT>
+static int prefill_t(const nnb200_gpt_config& c, const float* P, const WT* Wt, uint8_t* ws, const int* tokens_host, int n, int start,
+                     float* logits_out, cudaStream_t s)
+{
+    const DecodeWs W = decode_ws(c);
+    int* tok = reinterpret_cast<int*>(ws + W.p_tok);
+    if (n < kPromptMin || !attention_prompt_supported(c.d_model / c.heads)) {
+        int* step = reinterpret_cast<int*>(ws + W.step);
+        for (int i = 0; i < n; ++i) {
+            decode_set_step_kernel<<<1, 1, 0, s>>>(step, tokens_host[i], start + i, start + i);
+            NNB_LAUNCH_CHECK();
+            NNB_TRY(forward_step_t<WT>(c, P, Wt, ws, step, logits_out, s));
+        }
+        return 0;
+    }
+    int rows = 0;
+    for (int i = 0; i < n; i += rows) {
+        rows = std::min(n - i, kPromptRows);
+        NNB_CUDA_CHECK(cudaMemcpyAsync(tok, tokens_host + i, static_cast<size_t>(rows) * 4, cudaMemcpyHostToDevice, s));
+        NNB_TRY(prompt_pass_t<WT>(c, P, Wt, ws, tok, start + i, rows, s));
+    }
+    const DecodeLayout L = decode_layout(c);
+    float* F = reinterpret_cast<float*>(ws);
+    return gemv<WT, 1>(Wt + L.lm_w, F + W.p_x / 4 + static_cast<size_t>(rows - 1) * c.d_model, P + L.lnf_g, L.lnf_b >= 0 ? P + L.lnf_b : nullptr,
+                       c.norm == 0 ? 1 : 0, P + L.lm_b, nullptr, logits_out ? logits_out : F + W.logits / 4, c.vocab, c.d_model, s);
+}
+
 }  // namespace nnb
 
 using namespace nnb;
@@ -317,6 +402,19 @@ int nnb200_gpt_forward_step(const nnb200_gpt_config* cfg, const float* params, c
     decode_set_step_kernel<<<1, 1, 0, to_stream(stream)>>>(step, token_id, pos, cur_len);
     NNB_LAUNCH_CHECK();
     return forward_step_any(cfg, params, params_bf16, ws, step, logits_out, to_stream(stream));
+}
+
+int nnb200_gpt_prefill(const nnb200_gpt_config* cfg, const float* params, const void* params_bf16, void* workspace, const int32_t* tokens_host,
+                       int n, int cur_len, float* logits_out, void* stream)
+{
+    if (nnb200_gpt_arena_elems(cfg) < 0 || !params || !workspace || !tokens_host) { fprintf(stderr, "nnb200_gpt_prefill: bad arguments\n"); return -1; }
+    NNB_ARG_CHECK(n >= 1 && cur_len >= 0 && n <= cfg->seq && cur_len <= cfg->seq - n, "the cache holds seq rows: [cur_len, cur_len + n) must lie in them");
+    uint8_t* ws = static_cast<uint8_t*>(workspace);
+    if (cfg->precision == 1) {
+        NNB_ARG_CHECK(params_bf16 != nullptr, "bf16 mode needs the bf16 parameter shadow");
+        return prefill_t<bf16>(*cfg, params, static_cast<const bf16*>(params_bf16), ws, tokens_host, n, cur_len, logits_out, to_stream(stream));
+    }
+    return prefill_t<float>(*cfg, params, params, ws, tokens_host, n, cur_len, logits_out, to_stream(stream));
 }
 
 int nnb200_gpt_decode_set_step(int32_t* step_dev, int token_id, int pos, int cur_len, void* stream)

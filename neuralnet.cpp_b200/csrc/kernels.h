@@ -116,6 +116,10 @@ template <typename T> int attention_fwd_simt(const T* qkv, T* out, float* lse, c
 template <typename T> int attention_bwd_simt(const T* qkv, const T* out, const T* dout, const float* lse, float* dvec,
                                              T* dqkv, const int* doc, int B, int S, int H, int dk, int alibi,
                                              cudaStream_t s);
+// n prompt rows (q | k | v side by side) at positions start .. start + n - 1 over caches that already hold rows [0, start + n)
+bool attention_prompt_supported(int dk);
+int attention_prompt(const float* qkv, const float* k_cache, const float* v_cache, float* out, int start, int n, int H, int dk, int alibi,
+                     cudaStream_t s);
 int attention_dvec_bf16(const bf16* out, const bf16* dout, float* dvec, int B, int S, int H, int dk, cudaStream_t s);
 bool attention_mma_supported(int dk, int d);
 // attention_tc.cu : tcgen05 forward (head size 64 or 128, seq a multiple of 128).  doc_ranges (may be null): the table

@@ -320,7 +320,8 @@ class GptTrainer:
             args = (C.byref(self._c), _ptr(self.params), _ptr(self.shadow), _ptr(ws), _ptr(self._step_dev), _ptr(logits))
             side = torch.cuda.Stream(device=self.device)
             side.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(side):                      # one plain run first: per-device launch attributes are set there
+            with torch.cuda.stream(side):                      # one plain run of this token first: per-device launch attributes are set there
+                call("nnb200_gpt_decode_set_step", _ptr(self._step_dev), int(token_id), int(pos), int(cur_len), _stream())
                 call("nnb200_gpt_forward_step_dev", *args, _stream())
             torch.cuda.current_stream().wait_stream(side)
             g = torch.cuda.CUDAGraph()
@@ -329,6 +330,19 @@ class GptTrainer:
             self._decode_graph = g
         call("nnb200_gpt_decode_set_step", _ptr(self._step_dev), int(token_id), int(pos), int(cur_len), _stream())
         self._decode_graph.replay()
+        return logits
+
+    def prefill(self, tokens: Sequence[int], cur_len: int = 0) -> torch.Tensor:
+        """The tokens of a prompt through the model at once, at cache rows and positions cur_len onwards (what
+        GPTModel::generate does with one forward_step per token, compute_layer.hpp:2975-2990).  Returns the last token's
+        (vocab,) fp32 logits, in the tensor forward_step returns."""
+        ws, logits = self._decode_state()
+        n = len(tokens)
+        if not (n >= 1 and 0 <= int(cur_len) and int(cur_len) + n <= self.cfg.seq):
+            raise ValueError("the rows [cur_len, cur_len + tokens) must lie in [0, seq)")
+        ids = np.ascontiguousarray(tokens, np.int32)
+        call("nnb200_gpt_prefill", C.byref(self._c), _ptr(self.params), _ptr(self.shadow), _ptr(ws), C.c_void_p(ids.ctypes.data), n,
+             int(cur_len), _ptr(logits), _stream())
         return logits
 
     def generate(self, prompt: Sequence[int], max_new_tokens: int, temperature: float = 1.0, eos_token_id: int = -1,
@@ -344,6 +358,10 @@ class GptTrainer:
 
         def fill(start):
             nonlocal cur_len, last
+            if len(context) - start >= 8:            # shorter ones are quicker a token at a time
+                last = self.prefill(context[start:], cur_len)
+                cur_len += len(context) - start
+                return
             for t in context[start:]:
                 last = self.forward_step(t, cur_len, cur_len)
                 cur_len += 1
