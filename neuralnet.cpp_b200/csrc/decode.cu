@@ -2,31 +2,34 @@
 // Follows GPTModel::forward_step / GPTBlock::forward_step / AttentionBase::forward_step of the reference
 // (compute_layer.hpp:2906-2950, 1426-1511; ALiBi bias of a step :2267-2290; rotary encoding of a step :964-988), which
 // issues about thirty engine primitives, four transposes of the whole cache and two host-built matrices per block and
-// token; here a block is five launches (six with rotary positions) and nothing of the cache is copied.
-// A single token is all matrix-vector work, bound by reading the weights once: the kernels are warp-per-output-row
-// products with 16-byte loads over bf16 weights (the shadow copy, in bf16 mode) or the fp32 master weights (check mode),
-// fp32 activations and an fp32 cache in both modes.  The normalisation before a projection and the activation before
-// fc2 are applied while the input vector is staged in shared memory (every block does it for itself: the vector is a
-// few KB), the attention over the cache is split over chunks of 32 cached rows per head, and the token id, position
-// and cache length are read from device memory, so that the launches of a token are the same every time and a caller
-// may replay them as a CUDA graph (nnb200_gpt_forward_step_dev).
+// token; here a block is five launches and nothing of the cache is copied.
+// A single token is all matrix-vector work over bf16 weights (the shadow copy, in bf16 mode) or the fp32 master weights
+// (check mode), fp32 activations and an fp32 cache in both modes.  What bounds it is not the weights' bytes (182 MB, 27 us
+// for the 12-layer benchmark model) but the chain of about sixty dependent kernels, each of which would wait for its
+// predecessor, then for its first loads.  So each is launched while its predecessor runs (programmatic dependent launch),
+// loads what does not depend on it - its first weights, the norm's scale, the cached keys and values - into registers,
+// and only then waits for it.  The normalisation before a projection is done while the input vector is staged in shared
+// memory (every block does it for itself: the vector is a few KB), the activation in fc1's epilogue, the rotation of Q
+// and K in the attention kernel.  Nothing may read, before its wait, what a kernel of the same token writes.
+// The token id, position and cache length are read from device memory, so that the launches of a token are the same
+// every time and a caller may replay them as a CUDA graph (nnb200_gpt_forward_step_dev).
 #include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "kernels.h"
 #include "nnb200.h"
+#include "tc_ptx.cuh"
 
 namespace nnb {
 
-struct DecodeWs { size_t kv, table, x, xn, qkv, att, xmid, h1, h2, logits, step, part, count, total;
+struct DecodeWs { size_t kv, table, x, qkv, att, xmid, h2, logits, step, total;
                   size_t p_tok, p_x, p_xn, p_qkv, p_att, p_mid, p_h1, p_h2, p_stat; };
 // Rows of a prompt that one pass takes (longer prompts go in several): enough to fill the GEMM's tiles, 60 MB of
 // activations for a model of width 1024.
 constexpr int kPromptRows = 1024;
 // Shorter prompts go through the single-token kernels: a pass costs about as much as several tokens whatever its length.
 constexpr int kPromptMin = 8;
-constexpr int kDecodeChunk = 32;                    // cached rows per attention block: a block is one round of loads, bound by their latency
 static DecodeWs decode_ws(const nnb200_gpt_config& c)
 {
     DecodeWs W;
@@ -35,12 +38,8 @@ static DecodeWs decode_ws(const nnb200_gpt_config& c)
     auto take = [&](size_t floats) { const size_t o = off; off = (off + floats * 4 + 255) / 256 * 256; return o; };
     W.kv = take(static_cast<size_t>(c.layers) * 2 * S * d);
     W.table = take(S * d);
-    W.x = take(d); W.xn = take(d); W.qkv = take(3 * d); W.att = take(d); W.xmid = take(d);
-    W.h1 = take(fc1); W.h2 = take(c.d_ff); W.logits = take(c.vocab);
-    const size_t chunks = (S + kDecodeChunk - 1) / kDecodeChunk;
+    W.x = take(d); W.qkv = take(3 * d); W.att = take(d); W.xmid = take(d); W.h2 = take(c.d_ff); W.logits = take(c.vocab);
     W.step = take(4);                                            // token id, position, cache length
-    W.part = take(static_cast<size_t>(c.heads) * chunks * (d / c.heads + 2));   // per (head, chunk): maximum, sum, weighted values
-    W.count = take(static_cast<size_t>(c.heads));               // chunks of a head that have finished (back to zero after each step)
     const size_t R = std::min<size_t>(S, kPromptRows);
     W.p_tok = take(R); W.p_x = take(R * d); W.p_xn = take(R * d); W.p_qkv = take(R * 3 * d); W.p_att = take(R * d); W.p_mid = take(R * d);
     W.p_h1 = take(R * fc1); W.p_h2 = take(R * c.d_ff); W.p_stat = take(2 * R);
@@ -53,179 +52,362 @@ __global__ void decode_set_step_kernel(int* __restrict__ step, int token, int po
     step[0] = token; step[1] = pos; step[2] = cur_len;
 }
 
-// x = token embedding (+ position row); pos_table: learned or sinusoidal rows, or null
+// programmatic dependent launch: let the next kernel of the stream start / wait until the one before has finished
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+static int launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = static_cast<unsigned>(cluster); at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    NNB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    NNB_LAUNCH_CHECK();
+    return 0;
+}
+
+// x = token embedding (+ position row); pos_table: learned or sinusoidal rows, or null.  The first kernel of a token: launched
+// without the dependent-launch attribute, so that it and everything behind it starts after all earlier work of the stream.
 __global__ void decode_embed_kernel(const float* __restrict__ tok_emb, const float* __restrict__ pos_table, const int* __restrict__ step,
                                     int vocab, float* __restrict__ x, int d)
 {
+    pdl_launch();
     const int id = step[0], pos = step[1];
     const bool ok = id >= 0 && id < vocab;                      // an id out of range looks up a zero row (cpu_engine.hpp:150-158)
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < d; c += gridDim.x * blockDim.x)
         x[c] = (ok ? tok_emb[static_cast<size_t>(id) * d + c] : 0.f) + (pos_table ? pos_table[static_cast<size_t>(pos) * d + c] : 0.f);
 }
 
-// y[o] = W[o, :] . f(x) + bias[o] (+ residual[o]); one warp per output row, 16-byte loads along the row.  The input
-// vector is staged in shared memory by every block, and f is applied on the way:
-//   PRE 0: f = identity;
-//   PRE 1: f = norm(x) * gamma (+ beta), eps 1e-5 inside the rsqrt (compute_layer.hpp:495, 687; LayerNorm when `layer`);
-//   PRE 2: x holds fc1's output: f = SwiGLU (gate * sigmoid(gate) * up, `in` values out of 2 * in; compute_layer.hpp:
-//          375-404) or QuickGeLU (:266-295) when `layer` is 0 / 1.
-template <typename WT, int PRE>
-__global__ void __launch_bounds__(256) gemv_kernel(const WT* __restrict__ W, const float* __restrict__ x, const float* __restrict__ gamma,
+// y[o] = act(W[o, :] . f(x) + bias[o]) (+ residual[o]); a warp per group of R rows, 16-byte loads along the rows, eight of
+// them in flight per lane, the first eight before the wait for the previous kernel.
+//   NORM: f = norm(x) * gamma (+ beta), eps 1e-5 inside the rsqrt (compute_layer.hpp:495, 687; LayerNorm when `layer`).
+//   ACT 1: SwiGLU, y[o] = gate * sigmoid(gate) * up of rows o and o + out (compute_layer.hpp:375-404), R = 2;
+//   ACT 2: QuickGeLU (:266-295).
+// R is 1 where there are too few rows for more than a warp each (latency), 4 for the LM head (12 us of bytes: fewer
+// stagings of x per row).
+template <typename WT, bool NORM, int R, int ACT>
+__global__ void __launch_bounds__(256, 3) gemv_kernel(const WT* __restrict__ W, const float* __restrict__ x, const float* __restrict__ gamma,
                                                    const float* __restrict__ beta, int layer, const float* __restrict__ bias,
                                                    const float* __restrict__ residual, float* __restrict__ y, int out, int in)
 {
-    constexpr int VN = Vec16<WT>::N;
-    extern __shared__ float xs[];                               // `in` floats
+    static_assert(ACT != 1 || R == 2, "SwiGLU takes a gate and an up row");
+    constexpr int VN = Vec16<WT>::N, NC = 8 / R;
+    extern __shared__ __align__(16) float xs[];                 // `in` floats
     __shared__ float red[32];
-    if (PRE == 1) {
-        float mean = 0.f;
-        for (int c = threadIdx.x; c < in; c += blockDim.x) xs[c] = x[c];          // one trip to global memory, the passes read the copy
-        __syncthreads();
+    const int t = threadIdx.x, lane = t & 31, first = blockIdx.x * 8 + (t >> 5), step = gridDim.x * 8;
+    const int units = ACT == 1 ? out : (out + R - 1) / R;
+    const bool vec = (in % VN) == 0;
+    const bool in_regs = NORM && (in & 3) == 0 && in <= 1024 &&
+                         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) & 15) == 0;
+    auto row = [&](int u, int r) { return ACT == 1 ? u + r * out : u * R + r; };
+    auto row_ok = [&](int u, int r) { return ACT == 1 || R == 1 || u * R + r < out; };
+    uint4 w[R][NC];                                             // as loaded; widened where used (eight values would take eight registers)
+    auto load = [&](int u, int c0) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const WT* p = W + static_cast<size_t>(row(u, r)) * in;
+#pragma unroll
+            for (int i = 0; i < NC; ++i) {
+                const int c = c0 + (i * 32 + lane) * VN;
+                if (c < in && row_ok(u, r)) w[r][i] = *reinterpret_cast<const uint4*>(p + c);
+            }
+        }
+    };
+    if (vec && first < units) load(first, 0);
+    float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f), b4 = g4;
+    if (in_regs && t * 4 < in) {
+        g4 = *reinterpret_cast<const float4*>(gamma + t * 4);
+        if (beta) b4 = *reinterpret_cast<const float4*>(beta + t * 4);
+    }
+    pdl_launch();
+    pdl_wait();
+    if (in_regs) {
+        const bool mine = t * 4 < in;
+        float4 v = mine ? *reinterpret_cast<const float4*>(x + t * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (layer) {
-            float sacc = 0.f;
-            for (int c = threadIdx.x; c < in; c += blockDim.x) sacc += xs[c];
-            mean = block_sum(sacc, red) / static_cast<float>(in);
-            __syncthreads();
+            const float mean = block_sum((v.x + v.y) + (v.z + v.w), red) / static_cast<float>(in);
+            if (mine) { v.x -= mean; v.y -= mean; v.z -= mean; v.w -= mean; }
         }
-        float q = 0.f;
-        for (int c = threadIdx.x; c < in; c += blockDim.x) { const float v = xs[c] - mean; q += v * v; }
-        const float rinv = rsqrtf(block_sum(q, red) / static_cast<float>(in) + 1e-5f);
-        for (int c = threadIdx.x; c < in; c += blockDim.x) xs[c] = (xs[c] - mean) * rinv * gamma[c] + (beta ? beta[c] : 0.f);
-    } else if (PRE == 2) {
-        for (int c = threadIdx.x; c < in; c += blockDim.x) {
-            if (layer == 0) { const float g = x[c]; xs[c] = g / (1.0f + expf(-g)) * x[in + c]; }
-            else { const float v = x[c]; xs[c] = v / (1.0f + expf(-1.702f * v)); }
-        }
+        const float rinv = rsqrtf(block_sum((v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w), red) / static_cast<float>(in) + 1e-5f);
+        if (mine) *reinterpret_cast<float4*>(xs + t * 4) = make_float4(v.x * rinv * g4.x + b4.x, v.y * rinv * g4.y + b4.y, v.z * rinv * g4.z + b4.z, v.w * rinv * g4.w + b4.w);
     } else {
-        for (int c = threadIdx.x; c < in; c += blockDim.x) xs[c] = x[c];
+        if ((in & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+#pragma unroll 4
+            for (int c = t * 4; c < in; c += 1024) *reinterpret_cast<float4*>(xs + c) = *reinterpret_cast<const float4*>(x + c);
+        } else {
+#pragma unroll 4
+            for (int c = t; c < in; c += 256) xs[c] = x[c];
+        }
+        if (NORM) {
+            float mean = 0.f;
+            __syncthreads();
+            if (layer) {
+                float sacc = 0.f;
+                for (int c = t; c < in; c += 256) sacc += xs[c];
+                mean = block_sum(sacc, red) / static_cast<float>(in);
+            }
+            float q = 0.f;
+            for (int c = t; c < in; c += 256) { const float v = xs[c] - mean; q += v * v; }
+            const float rinv = rsqrtf(block_sum(q, red) / static_cast<float>(in) + 1e-5f);
+            for (int c = t; c < in; c += 256) xs[c] = (xs[c] - mean) * rinv * gamma[c] + (beta ? beta[c] : 0.f);
+        }
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
-    for (int o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; o < out; o += warps) {
-        const WT* w = W + static_cast<size_t>(o) * in;
-        float acc = 0.f;
-        if ((in % VN) == 0) {
-            for (int c = lane * VN; c < in; c += 32 * VN) {
-                const Vec16<WT> v = ld16(w + c);
+    for (int u = first; u < units; u += step) {
+        float acc[R];
 #pragma unroll
-                for (int k = 0; k < VN; ++k) acc = fmaf(to_f32(v.v[k]), xs[c + k], acc);
+        for (int r = 0; r < R; ++r) acc[r] = 0.f;
+        if (vec) {
+            for (int c0 = 0; c0 < in; c0 += NC * 32 * VN) {
+                if (c0 > 0 || u != first) load(u, c0);
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int i = 0; i < NC; ++i) asm volatile("" : "+r"(w[r][i].x), "+r"(w[r][i].y), "+r"(w[r][i].z), "+r"(w[r][i].w));
+#pragma unroll
+                for (int i = 0; i < NC; ++i) {
+                    const int c = c0 + (i * 32 + lane) * VN;
+                    if (c < in) {
+#pragma unroll
+                        for (int k = 0; k < VN; k += 4) {
+                            const float4 f = *reinterpret_cast<const float4*>(xs + c + k);
+#pragma unroll
+                            for (int r = 0; r < R; ++r) {
+                                if (!row_ok(u, r)) continue;
+                                Vec16<WT> v;
+                                *reinterpret_cast<uint4*>(&v) = w[r][i];
+                                acc[r] = fmaf(to_f32(v.v[k]), f.x, acc[r]);
+                                acc[r] = fmaf(to_f32(v.v[k + 1]), f.y, acc[r]);
+                                acc[r] = fmaf(to_f32(v.v[k + 2]), f.z, acc[r]);
+                                acc[r] = fmaf(to_f32(v.v[k + 3]), f.w, acc[r]);
+                            }
+                        }
+                    }
+                }
             }
         } else {
-            for (int c = lane; c < in; c += 32) acc = fmaf(to_f32(w[c]), xs[c], acc);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (!row_ok(u, r)) continue;
+                const WT* p = W + static_cast<size_t>(row(u, r)) * in;
+                for (int c = lane; c < in; c += 32) acc[r] = fmaf(to_f32(p[c]), xs[c], acc[r]);
+            }
         }
-        acc = warp_sum(acc);
-        if (lane == 0) y[o] = acc + (bias ? bias[o] : 0.f) + (residual ? residual[o] : 0.f);
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r] = warp_sum(acc[r]);
+        if (lane != 0) continue;
+        if (ACT == 1) {
+            const float g = acc[0] + bias[u];
+            y[u] = g / (1.0f + expf(-g)) * (acc[R - 1] + bias[u + out]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int o = u * R + r;
+                if (!row_ok(u, r)) continue;
+                float v = acc[r] + bias[o];
+                if (ACT == 2) v = v / (1.0f + expf(-1.702f * v));
+                y[o] = v + (residual ? residual[o] : 0.f);
+            }
+        }
     }
 }
 
-// Rotary encoding of the Q and K thirds of one token's qkv vector at position `pos` (table: cos (seq, dk/2) then sin)
-__global__ void decode_rope_kernel(float* __restrict__ qkv, const float* __restrict__ table, const int* __restrict__ step, int seq, int heads,
-                                   int dk)
+// Attention of one token over the cache: a cluster of eight blocks per head, cached row j on lane group j modulo all the groups
+// of the cluster (LPR lanes carry a row, NV 16-byte vectors each), B rows in flight per group.  All cached rows but the
+// token's own were written by earlier tokens, so the first B keys and values are loaded before the wait.  The token's key
+// and value are appended to the cache on the way.  Scores q_h . k_j / sqrt(dk) - slope_h (cur_len - j), softmax kept online
+// per group, groups merged by shuffles, warps through shared memory and blocks through the cluster's shared memory, in a
+// fixed order.  The grid is the same for every cache length.
+// 12 heads of 64 behind 900 tokens: bound by the chain wait - scores - merge.  (Blocks of 32 rows that left partial results
+// in global memory and elected the last one to merge them took 22.6 us.)
+template <int LPR, int NV, bool VEC>
+__global__ void __launch_bounds__(256) decode_attn_kernel(const float* __restrict__ qkv, float* __restrict__ kc, float* __restrict__ vc,
+                                                          float* __restrict__ out, const float* __restrict__ rope, const int* __restrict__ step,
+                                                          int seq, int d, int dk, int heads, int alibi, float scale)
 {
-    const int pos = step[2];                                    // the rotation of a step is by the cache row it lands in
-    const int half = dk / 2, n = 2 * heads * half;
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x) {
-        const int j = w % half, h = (w / half) % heads, which = w / (half * heads);
-        float* lo = qkv + which * heads * dk + h * dk + j;
-        const float c = table[static_cast<size_t>(pos) * half + j], sn = table[static_cast<size_t>(seq) * half + static_cast<size_t>(pos) * half + j];
-        const float a = lo[0], b = lo[half];
-        lo[0] = a * c - b * sn;
-        lo[half] = b * c + a * sn;
-    }
-}
-
-// Attention of one token over the cache, split over chunks of kDecodeChunk cached rows: block (head, chunk).  The block
-// of chunk cur_len / kDecodeChunk appends this token's key and value to the cache (row cur_len) first.  Every block
-// computes the scores of its rows (q_h . k_j / sqrt(dk) - slope_h (cur_len - j)), their maximum, the sum of the
-// exponentials against it and the weighted values, and leaves them as a partial; the block of a head that finishes last
-// merges the head's partials in chunk order (the same order whatever the finishing order) and writes out_h.
-// Chunks beyond the cache length leave at once: the grid is the same for every cache length.
-__global__ void __launch_bounds__(128) decode_attn_kernel(const float* __restrict__ qkv, float* __restrict__ kc, float* __restrict__ vc,
-                                                          float* __restrict__ out, const int* __restrict__ step, float* __restrict__ part,
-                                                          int* __restrict__ count, int d, int dk, int heads, int alibi, float scale)
-{
-    __shared__ float sc[kDecodeChunk];
-    __shared__ float red[32];
-    __shared__ float qs[256];
-    __shared__ float ov[2][256];
-    __shared__ int last;
-    const int h = blockIdx.x, chunk = blockIdx.y, nchunks_max = gridDim.y;
-    const int cur_len = step[2], n = cur_len + 1;
-    const int j0 = chunk * kDecodeChunk;
-    if (j0 >= n) return;
-    const int nchunks = (n + kDecodeChunk - 1) / kDecodeChunk;
-    const int rows = min(kDecodeChunk, n - j0);
-    for (int c = threadIdx.x; c < dk; c += blockDim.x) qs[c] = qkv[h * dk + c];
-    if (cur_len >= j0 && cur_len < j0 + kDecodeChunk)
-        for (int c = threadIdx.x; c < dk; c += blockDim.x) {
-            kc[static_cast<size_t>(cur_len) * d + h * dk + c] = qkv[d + h * dk + c];
-            vc[static_cast<size_t>(cur_len) * d + h * dk + c] = qkv[2 * d + h * dk + c];
+    constexpr int B = 8 / NV, G = 256 / LPR, RANKS = 8, DMAX = LPR * NV * 4;
+    __shared__ float wm[8], wl[8];
+    __shared__ __align__(16) float wo[8][DMAX];
+    __shared__ float part[DMAX + 2];                            // this block's maximum, sum and weighted values
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, sub = t % LPR, h = blockIdx.x / RANKS;
+    const int rank = static_cast<int>(cluster_ctarank()), g0 = rank * G + t / LPR;
+    const int cur = step[2], n = cur + 1;
+    const size_t head = static_cast<size_t>(h) * dk;
+    auto fetch = [&](const float* p, float (&v)[NV * 4]) {      // this lane's columns of a row; zero beyond dk
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = (i * LPR + sub) * 4;
+            if (VEC) {
+                const float4 f = c < dk ? *reinterpret_cast<const float4*>(p + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[i * 4] = f.x; v[i * 4 + 1] = f.y; v[i * 4 + 2] = f.z; v[i * 4 + 3] = f.w;
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[i * 4 + k] = c + k < dk ? p[c + k] : 0.f;
+            }
         }
-    __syncthreads();
+    };
+    float kr[B][NV * 4], vr[B][NV * 4];
+    auto load = [&](int j0) {
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int j = j0 + b * (RANKS * G);
+            if (j < cur) {
+                fetch(kc + static_cast<size_t>(j) * d + head, kr[b]);
+                fetch(vc + static_cast<size_t>(j) * d + head, vr[b]);
+            }
+        }
+    };
+    load(g0);
+    pdl_launch();
+    pdl_wait();
+    // q or the new k: rotated with rotary positions by the cache row it lands in (table: cos (seq, dk/2), then sin)
+    auto rotated = [&](const float* p, float (&v)[NV * 4]) {
+        fetch(p, v);
+        if (!rope) return;
+        const int half = dk / 2;
+        const float *cs = rope + static_cast<size_t>(cur) * half, *sn = rope + (static_cast<size_t>(seq) + cur) * half;
+#pragma unroll
+        for (int i = 0; i < NV * 4; ++i) {
+            const int c = ((i / 4) * LPR + sub) * 4 + i % 4;
+            if (c < half) v[i] = v[i] * cs[c] - p[c + half] * sn[c];
+            else if (c < dk) v[i] = v[i] * cs[c - half] + p[c - half] * sn[c - half];
+        }
+    };
+    float q[NV * 4], o[NV * 4];
+    rotated(qkv + head, q);
+#pragma unroll
+    for (int i = 0; i < NV * 4; ++i) o[i] = 0.f;
     const float slope = alibi ? exp2f(-8.0f * static_cast<float>(h) / static_cast<float>(heads)) : 0.f;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    float mx = -INFINITY;
-#pragma unroll 8
-    for (int r = warp; r < rows; r += nwarps) {
-        const int j = j0 + r;
-        const float* kr = kc + static_cast<size_t>(j) * d + h * dk;
-        float acc = 0.f;
-        for (int c = lane; c < dk; c += 32) acc = fmaf(qs[c], kr[c], acc);
-        acc = warp_sum(acc) * scale - slope * static_cast<float>(cur_len - j);
-        if (lane == 0) sc[r] = acc;
-        mx = fmaxf(mx, acc);
-    }
-    mx = block_max(mx, red);
-    __syncthreads();
-    float den = 0.f;
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) { const float e = expf(sc[r] - mx); sc[r] = e; den += e; }
-    den = block_sum(den, red);
-    __syncthreads();
-    // weighted values: thread (column, half of the rows); head sizes up to 256 with 128 threads need one or more rounds
-    float* my = part + (static_cast<size_t>(h) * nchunks_max + chunk) * (dk + 2);
-    for (int c0 = 0; c0 < dk; c0 += 64) {
-        const int c = c0 + (threadIdx.x & 63), half = threadIdx.x >> 6;
-        float acc = 0.f;
-        if (c < dk) {
-#pragma unroll 8
-            for (int r = half; r < rows; r += 2) acc = fmaf(sc[r], vc[static_cast<size_t>(j0 + r) * d + h * dk + c], acc);
+    float m = -INFINITY, l = 0.f;
+    for (int j0 = g0; j0 - t / LPR % (32 / LPR) < n; j0 += B * RANKS * G) {     // the same number of rounds for all groups of a warp
+        if (j0 != g0) load(j0);
+        float s[B];
+        float mx = m;
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const int j = j0 + b * (RANKS * G);
+            if (j == cur) {
+                rotated(qkv + d + head, kr[b]);
+                fetch(qkv + 2 * d + head, vr[b]);
+#pragma unroll
+                for (int i = 0; i < NV * 4; ++i) {
+                    const int c = ((i / 4) * LPR + sub) * 4 + i % 4;
+                    if (c < dk) {
+                        kc[static_cast<size_t>(cur) * d + head + c] = kr[b][i];
+                        vc[static_cast<size_t>(cur) * d + head + c] = vr[b][i];
+                    }
+                }
+            }
+            float a = 0.f;
+            if (j < n) {
+#pragma unroll
+                for (int i = 0; i < NV * 4; ++i) a = fmaf(q[i], kr[b][i], a);
+            }
+#pragma unroll
+            for (int w = LPR / 2; w > 0; w >>= 1) a += __shfl_xor_sync(0xffffffffu, a, w);
+            s[b] = j < n ? a * scale - slope * static_cast<float>(cur - j) : -INFINITY;
+            mx = fmaxf(mx, s[b]);
         }
-        ov[half][c0 + (threadIdx.x & 63)] = acc;
-        __syncthreads();
-        if (half == 0 && c < dk) my[2 + c] = ov[0][c] + ov[1][c];
-        __syncthreads();
+        const float ref = mx == -INFINITY ? 0.f : mx, back = expf(m - ref);
+        m = mx;
+        l *= back;
+#pragma unroll
+        for (int i = 0; i < NV * 4; ++i) o[i] *= back;
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            if (j0 + b * (RANKS * G) >= n) break;
+            const float e = expf(s[b] - ref);
+            l += e;
+#pragma unroll
+            for (int i = 0; i < NV * 4; ++i) o[i] = fmaf(e, vr[b][i], o[i]);
+        }
     }
-    if (threadIdx.x == 0) { my[0] = mx; my[1] = den; }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(count + h, 1) == nchunks - 1);
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    if (threadIdx.x == 0) count[h] = 0;
-    const float* hp = part + static_cast<size_t>(h) * nchunks_max * (dk + 2);
-    float gm = -INFINITY;
-    for (int k = 0; k < nchunks; ++k) gm = fmaxf(gm, __ldcg(hp + static_cast<size_t>(k) * (dk + 2)));
-    float gden = 0.f;
-    for (int k = 0; k < nchunks; ++k) gden += __ldcg(hp + static_cast<size_t>(k) * (dk + 2) + 1) * expf(__ldcg(hp + static_cast<size_t>(k) * (dk + 2)) - gm);
-    const float inv = 1.0f / gden;
-    for (int c = threadIdx.x; c < dk; c += blockDim.x) {
-        float acc = 0.f;
-        for (int k = 0; k < nchunks; ++k)
-            acc = fmaf(__ldcg(hp + static_cast<size_t>(k) * (dk + 2) + 2 + c), expf(__ldcg(hp + static_cast<size_t>(k) * (dk + 2)) - gm), acc);
-        out[h * dk + c] = acc * inv;
+#pragma unroll
+    for (int w = LPR; w < 32; w <<= 1) {                        // groups of a warp
+        const float om = __shfl_xor_sync(0xffffffffu, m, w), nm = fmaxf(m, om), ref = nm == -INFINITY ? 0.f : nm;
+        const float a = expf(m - ref), b = expf(om - ref);
+        l = l * a + __shfl_xor_sync(0xffffffffu, l, w) * b;
+#pragma unroll
+        for (int i = 0; i < NV * 4; ++i) o[i] = o[i] * a + __shfl_xor_sync(0xffffffffu, o[i], w) * b;
+        m = nm;
     }
+    if (lane == 0) { wm[warp] = m; wl[warp] = l; }
+    if (lane < LPR) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) *reinterpret_cast<float4*>(&wo[warp][(i * LPR + sub) * 4]) = make_float4(o[i * 4], o[i * 4 + 1], o[i * 4 + 2], o[i * 4 + 3]);
+    }
+    __syncthreads();
+    {                                                           // warps of the block
+        float bm = wm[0];
+#pragma unroll
+        for (int w = 1; w < 8; ++w) bm = fmaxf(bm, wm[w]);
+        const float ref = bm == -INFINITY ? 0.f : bm;
+        if (t < DMAX) {
+            float bl = 0.f, a = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) { const float e = expf(wm[w] - ref); bl += wl[w] * e; a = fmaf(wo[w][t], e, a); }
+            part[2 + t] = a;
+            if (t == 0) { part[0] = bm; part[1] = bl; }
+        }
+    }
+    cluster_sync_all();
+    const int cols = (dk + RANKS - 1) / RANKS, c = rank * cols + t;
+    if (t < cols && c < dk) {                                   // blocks of the cluster: each finishes its share of the columns
+        const uint32_t base = smem_u32(part);
+        float pm[RANKS], pl[RANKS], po[RANKS], gm = -INFINITY, gl = 0.f, a = 0.f;
+#pragma unroll
+        for (int r = 0; r < RANKS; ++r) {
+            const uint32_t p = mapa_shared(base, r);
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(pm[r]) : "r"(p) : "memory");
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(pl[r]) : "r"(p + 4) : "memory");
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(po[r]) : "r"(p + 8 + 4 * c) : "memory");
+        }
+#pragma unroll
+        for (int r = 0; r < RANKS; ++r) gm = fmaxf(gm, pm[r]);
+        const float ref = gm == -INFINITY ? 0.f : gm;
+#pragma unroll
+        for (int r = 0; r < RANKS; ++r) { const float e = expf(pm[r] - ref); gl += pl[r] * e; a = fmaf(po[r], e, a); }
+        out[head + c] = a / gl;
+    }
+    cluster_sync_all();                                         // nobody's shared memory goes while a peer reads it
 }
 
-template <typename WT, int PRE>
+template <typename WT, bool NORM, int R, int ACT>
 static int gemv(const WT* W, const float* x, const float* gamma, const float* beta, int layer, const float* bias, const float* residual,
                 float* y, int out, int in, cudaStream_t s)
 {
     NNB_ARG_CHECK(static_cast<size_t>(in) * sizeof(float) <= 48 * 1024, "input vector too long for the decode matrix-vector kernel");
-    gemv_kernel<WT, PRE><<<grid_for(static_cast<long long>(out) * 32, 256), 256, static_cast<size_t>(in) * sizeof(float), s>>>(
-        W, x, gamma, beta, layer, bias, residual, y, out, in);
-    NNB_LAUNCH_CHECK();
-    return 0;
+    const long long units = ACT == 1 ? out : ceil_div(out, R);
+    return launch_dependent(gemv_kernel<WT, NORM, R, ACT>, dim3(grid_for(units, 8)), 256, static_cast<size_t>(in) * sizeof(float), 1, s, W, x, gamma,
+                            beta, layer, bias, residual, y, out, in);
+}
+
+static int decode_attention(const float* qkv, float* kc, float* vc, float* out, const float* rope, const int* step, const nnb200_gpt_config& c, cudaStream_t s)
+{
+    const int d = c.d_model, dk = d / c.heads;
+    const dim3 grid(static_cast<unsigned>(c.heads) * 8);
+    auto go = [&](auto* kernel) {
+        return launch_dependent(kernel, grid, 256, 0, 8, s, qkv, kc, vc, out, rope, step, c.seq, d, dk, c.heads, c.pos == 2 ? 1 : 0,
+                                1.0f / sqrtf(static_cast<float>(dk)));
+    };
+    if (dk % 4 == 0 && ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0) {
+        if (dk <= 32) return go(decode_attn_kernel<8, 1, true>);
+        if (dk <= 64) return go(decode_attn_kernel<16, 1, true>);
+        if (dk <= 128) return go(decode_attn_kernel<32, 1, true>);
+        return go(decode_attn_kernel<32, 2, true>);
+    }
+    if (dk <= 128) return go(decode_attn_kernel<32, 1, false>);
+    return go(decode_attn_kernel<32, 2, false>);
 }
 
 // `step` (device): token id, position, cache length
@@ -235,7 +417,7 @@ static int forward_step_t(const nnb200_gpt_config& c, const float* P, const WT* 
 {
     const DecodeLayout L = decode_layout(c);
     const DecodeWs W = decode_ws(c);
-    const int d = c.d_model, ff = c.d_ff, fc1 = c.act == 1 ? 2 * ff : ff, dk = d / c.heads;
+    const int d = c.d_model, ff = c.d_ff, dk = d / c.heads;
     const int ln = c.norm == 0 ? 1 : 0;
     NNB_ARG_CHECK(dk <= 256, "head size above 256");
     auto F = [&](size_t off) { return reinterpret_cast<float*>(ws + off); };
@@ -246,26 +428,20 @@ static int forward_step_t(const nnb200_gpt_config& c, const float* P, const WT* 
     decode_embed_kernel<<<grid_for(d, 256), 256, 0, s>>>(P + L.tok_emb, pos_table, step, c.vocab, F(W.x), d);
     NNB_LAUNCH_CHECK();
     const size_t layer_kv = static_cast<size_t>(2) * c.seq * d;
-    const dim3 attn_grid(static_cast<unsigned>(c.heads), static_cast<unsigned>((c.seq + kDecodeChunk - 1) / kDecodeChunk));
     float* x = F(W.x);
     float* xmid = F(W.xmid);
     for (int l = 0; l < c.layers; ++l) {
         const DecodeLayer& lp = L.layers[l];
         float* kc = F(W.kv) + static_cast<size_t>(l) * layer_kv;
         float* vc = kc + static_cast<size_t>(c.seq) * d;
-        NNB_TRY((gemv<WT, 1>(Wt + lp.wqkv, x, P + lp.g1, PB(lp.be1), ln, P + lp.bqkv, nullptr, F(W.qkv), 3 * d, d, s)));
-        if (c.pos == 3) {
-            decode_rope_kernel<<<grid_for(static_cast<long long>(c.heads) * dk, 256), 256, 0, s>>>(F(W.qkv), F(W.table), step, c.seq, c.heads, dk);
-            NNB_LAUNCH_CHECK();
-        }
-        decode_attn_kernel<<<attn_grid, 128, 0, s>>>(F(W.qkv), kc, vc, F(W.att), step, F(W.part), reinterpret_cast<int*>(F(W.count)), d, dk,
-                                                     c.heads, c.pos == 2 ? 1 : 0, 1.0f / sqrtf(static_cast<float>(dk)));
-        NNB_LAUNCH_CHECK();
-        NNB_TRY((gemv<WT, 0>(Wt + lp.wo, F(W.att), nullptr, nullptr, 0, P + lp.bo, x, xmid, d, d, s)));          // + residual (GPTBlock::forward_step)
-        NNB_TRY((gemv<WT, 1>(Wt + lp.w1, xmid, P + lp.g2, PB(lp.be2), ln, P + lp.b1, nullptr, F(W.h1), fc1, d, s)));
-        NNB_TRY((gemv<WT, 2>(Wt + lp.w2, F(W.h1), nullptr, nullptr, c.act == 1 ? 0 : 1, P + lp.b2, xmid, x, d, ff, s)));   // + residual
+        NNB_TRY((gemv<WT, true, 1, 0>(Wt + lp.wqkv, x, P + lp.g1, PB(lp.be1), ln, P + lp.bqkv, nullptr, F(W.qkv), 3 * d, d, s)));
+        NNB_TRY(decode_attention(F(W.qkv), kc, vc, F(W.att), c.pos == 3 ? F(W.table) : nullptr, step, c, s));
+        NNB_TRY((gemv<WT, false, 1, 0>(Wt + lp.wo, F(W.att), nullptr, nullptr, 0, P + lp.bo, x, xmid, d, d, s)));          // + residual (GPTBlock::forward_step)
+        if (c.act == 1) NNB_TRY((gemv<WT, true, 2, 1>(Wt + lp.w1, xmid, P + lp.g2, PB(lp.be2), ln, P + lp.b1, nullptr, F(W.h2), ff, d, s)));
+        else NNB_TRY((gemv<WT, true, 1, 2>(Wt + lp.w1, xmid, P + lp.g2, PB(lp.be2), ln, P + lp.b1, nullptr, F(W.h2), ff, d, s)));
+        NNB_TRY((gemv<WT, false, 1, 0>(Wt + lp.w2, F(W.h2), nullptr, nullptr, 0, P + lp.b2, xmid, x, d, ff, s)));   // + residual
     }
-    return gemv<WT, 1>(Wt + L.lm_w, x, P + L.lnf_g, PB(L.lnf_b), ln, P + L.lm_b, nullptr, logits_out ? logits_out : F(W.logits), c.vocab, d, s);
+    return gemv<WT, true, 4, 0>(Wt + L.lm_w, x, P + L.lnf_g, PB(L.lnf_b), ln, P + L.lm_b, nullptr, logits_out ? logits_out : F(W.logits), c.vocab, d, s);
 }
 
 // Y[n, out] = X[n, in] W[out, in]^T + bias (+ residual), fp32 rows times fp32 or bf16 weights
@@ -322,7 +498,8 @@ static int prefill_t(const nnb200_gpt_config& c, const float* P, const WT* Wt, u
 {
     const DecodeWs W = decode_ws(c);
     int* tok = reinterpret_cast<int*>(ws + W.p_tok);
-    if (n < kPromptMin || !attention_prompt_supported(c.d_model / c.heads)) {
+    const bool aligned = ((reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(P)) & 15) == 0;      // the row kernels' vectors
+    if (n < kPromptMin || !aligned || !attention_prompt_supported(c.d_model / c.heads)) {
         int* step = reinterpret_cast<int*>(ws + W.step);
         for (int i = 0; i < n; ++i) {
             decode_set_step_kernel<<<1, 1, 0, s>>>(step, tokens_host[i], start + i, start + i);
@@ -339,7 +516,7 @@ static int prefill_t(const nnb200_gpt_config& c, const float* P, const WT* Wt, u
     }
     const DecodeLayout L = decode_layout(c);
     float* F = reinterpret_cast<float*>(ws);
-    return gemv<WT, 1>(Wt + L.lm_w, F + W.p_x / 4 + static_cast<size_t>(rows - 1) * c.d_model, P + L.lnf_g, L.lnf_b >= 0 ? P + L.lnf_b : nullptr,
+    return gemv<WT, true, 4, 0>(Wt + L.lm_w, F + W.p_x / 4 + static_cast<size_t>(rows - 1) * c.d_model, P + L.lnf_g, L.lnf_b >= 0 ? P + L.lnf_b : nullptr,
                        c.norm == 0 ? 1 : 0, P + L.lm_b, nullptr, logits_out ? logits_out : F + W.logits / 4, c.vocab, c.d_model, s);
 }
 
@@ -373,7 +550,6 @@ int nnb200_gpt_decode_init(const nnb200_gpt_config* cfg, void* workspace, void* 
                 tab[static_cast<size_t>(pos) * d + i] = (i % 2 == 0) ? std::sin(angle) : std::cos(angle);
             }
     }
-    NNB_CUDA_CHECK(cudaMemsetAsync(static_cast<uint8_t*>(workspace) + W.count, 0, static_cast<size_t>(cfg->heads) * sizeof(int), to_stream(stream)));
     if (!tab.empty()) {
         NNB_CUDA_CHECK(cudaMemcpyAsync(static_cast<uint8_t*>(workspace) + W.table, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice, to_stream(stream)));
         NNB_CUDA_CHECK(cudaStreamSynchronize(to_stream(stream)));          // `tab` is pageable host memory about to go away
