@@ -1,4 +1,6 @@
-"""The row kernels of the norms where the row's last vectors go to some lanes only."""
+"""The row kernels of the norms where the row's last vectors go to some lanes only, and the sum of squares at every remainder."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -28,3 +30,16 @@ def test_training_step_of_a_width_that_leaves_lanes_empty(d, precision, norm):
     got = tr.get_grads()
     # fp32: rounding of sums of up to 504 terms; bf16: about twenty tensors rounded by at most 2^-9 each on the way, partly cancelling
     assert global_rel_err(got, want, key_bias_indices(cfg)) < (1e-5 if precision == 0 else 3e-2)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 1023, 4097, 592 * 256 * 16, 592 * 256 * 16 + 4099])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_sum_of_squares(n, offset):
+    import torch
+    from tests import gpu_util as g
+    t = torch.randn(n + offset, device="cuda")[offset:]
+    scratch = torch.zeros(int(g.call("nnb200_sumsq_scratch_floats")), device="cuda")
+    out = torch.zeros(4, device="cuda")
+    g.call("nnb200_grad_norm_clip", g.ptr(t), n, C.c_float(0.5), C.c_float(1.0), g.ptr(scratch), g.ptr(out), g.stream())
+    # positive terms: sums of at most ~100 per thread and 600 per block, each within eps / 2
+    assert np.isclose(float(out[1]), 0.5 * float(t.double().norm()), rtol=1e-5)
