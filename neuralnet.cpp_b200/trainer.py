@@ -315,22 +315,29 @@ class GptTrainer:
             call("nnb200_gpt_forward_step", C.byref(self._c), _ptr(self.params), _ptr(self.shadow), _ptr(ws), int(token_id), int(pos),
                  int(cur_len), _ptr(logits), _stream())
             return logits
-        if getattr(self, "_decode_graph", None) is None:
-            self._step_dev = torch.zeros(4, dtype=torch.int32, device=self.device)
-            args = (C.byref(self._c), _ptr(self.params), _ptr(self.shadow), _ptr(ws), _ptr(self._step_dev), _ptr(logits))
-            side = torch.cuda.Stream(device=self.device)
-            side.wait_stream(torch.cuda.current_stream())
-            with torch.cuda.stream(side):                      # one plain run of this token first: per-device launch attributes are set there
-                call("nnb200_gpt_decode_set_step", _ptr(self._step_dev), int(token_id), int(pos), int(cur_len), _stream())
-                call("nnb200_gpt_forward_step_dev", *args, _stream())
-            torch.cuda.current_stream().wait_stream(side)
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
-                call("nnb200_gpt_forward_step_dev", *args, _stream())
-            self._decode_graph = g
+        self._capture_step(token_id, pos, cur_len)
         call("nnb200_gpt_decode_set_step", _ptr(self._step_dev), int(token_id), int(pos), int(cur_len), _stream())
         self._decode_graph.replay()
         return logits
+
+    def _capture_step(self, token_id: int, pos: int, cur_len: int):
+        """Captures the launches of forward_step, once.  Runs the given token first (lazy loading of kernels is not for a
+        capture), which writes no cache row but cur_len."""
+        if getattr(self, "_decode_graph", None) is not None:
+            return
+        ws, logits = self._decode_state()
+        self._step_dev = torch.zeros(4, dtype=torch.int32, device=self.device)
+        args = (C.byref(self._c), _ptr(self.params), _ptr(self.shadow), _ptr(ws), _ptr(self._step_dev), _ptr(logits))
+        side = torch.cuda.Stream(device=self.device)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            call("nnb200_gpt_decode_set_step", _ptr(self._step_dev), int(token_id), int(pos), int(cur_len), _stream())
+            call("nnb200_gpt_forward_step_dev", *args, _stream())
+        torch.cuda.current_stream().wait_stream(side)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            call("nnb200_gpt_forward_step_dev", *args, _stream())
+        self._decode_graph = g
 
     def prefill(self, tokens: Sequence[int], cur_len: int = 0) -> torch.Tensor:
         """The tokens of a prompt through the model at once, at cache rows and positions cur_len onwards (what
@@ -341,6 +348,7 @@ class GptTrainer:
         if not (n >= 1 and 0 <= int(cur_len) and int(cur_len) + n <= self.cfg.seq):
             raise ValueError("the rows [cur_len, cur_len + tokens) must lie in [0, seq)")
         ids = np.ascontiguousarray(tokens, np.int32)
+        self._capture_step(ids[0], cur_len, cur_len)         # not in the first token behind the prompt; row cur_len is written again below
         call("nnb200_gpt_prefill", C.byref(self._c), _ptr(self.params), _ptr(self.shadow), _ptr(ws), C.c_void_p(ids.ctypes.data), n,
              int(cur_len), _ptr(logits), _stream())
         return logits
