@@ -351,7 +351,7 @@ int nnb200_gpt_forward_step(const nnb200_gpt_config* cfg, const float* params, c
  * replay it per token after updating step_dev.  No counterpart in the reference, which builds its step on the host. */
 int nnb200_gpt_forward_step_dev(const nnb200_gpt_config* cfg, const float* params, const void* params_bf16, void* workspace,
                                 const int32_t* step_dev, float* logits_out, void* stream);
-/* A whole prompt at once: tokens_host (host memory, read before the call returns) go to cache rows and positions
+/* A whole prompt at once: tokens_host (host memory of any kind, read before the call returns) go to cache rows and positions
  * [cur_len, cur_len + n), attending to the rows before them, and logits_out (device, vocab fp32; null = kept in the
  * workspace) receives the last token's logits: what n calls of nnb200_gpt_forward_step leave. */
 int nnb200_gpt_prefill(const nnb200_gpt_config* cfg, const float* params, const void* params_bf16, void* workspace,

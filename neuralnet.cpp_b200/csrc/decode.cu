@@ -54,6 +54,27 @@ __global__ void decode_set_step_kernel(int* __restrict__ step, int token, int po
     step[0] = token; step[1] = pos; step[2] = cur_len;
 }
 
+// Prompt ids travel as kernel parameters: the caller's buffer is read before the launch call returns, whatever kind of host
+// memory it is (a copy from page-locked memory would read it when the stream gets there).
+struct PromptIds { int id[512]; };
+__global__ void decode_set_prompt_kernel(int* __restrict__ tok, const __grid_constant__ PromptIds ids, int n)
+{
+    if (static_cast<int>(threadIdx.x) < n) tok[threadIdx.x] = ids.id[threadIdx.x];
+}
+static int set_prompt(int* tok, const int* tokens_host, int n, cudaStream_t s)
+{
+    constexpr int kIds = static_cast<int>(sizeof(PromptIds) / sizeof(int));
+    for (int i = 0; i < n; i += kIds) {
+        const int k = std::min(n - i, kIds);
+        PromptIds ids;
+        std::copy_n(tokens_host + i, k, ids.id);
+        std::fill(ids.id + k, ids.id + kIds, 0);
+        decode_set_prompt_kernel<<<1, kIds, 0, s>>>(tok + i, ids, k);
+        NNB_LAUNCH_CHECK();
+    }
+    return 0;
+}
+
 // programmatic dependent launch: let the next kernel of the stream start / wait until the one before has finished
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -514,7 +535,7 @@ static int prefill_t(const nnb200_gpt_config& c, const float* P, const WT* Wt, u
     int rows = 0;
     for (int i = 0; i < n; i += rows) {
         rows = std::min(n - i, kPromptRows);
-        NNB_CUDA_CHECK(cudaMemcpyAsync(tok, tokens_host + i, static_cast<size_t>(rows) * 4, cudaMemcpyHostToDevice, s));
+        NNB_TRY(set_prompt(tok, tokens_host + i, rows, s));
         NNB_TRY(prompt_pass_t<WT>(c, P, Wt, ws, tok, start + i, rows, s));
     }
     const DecodeLayout L = decode_layout(c);

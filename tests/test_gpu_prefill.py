@@ -51,3 +51,23 @@ def test_prefill_refuses_rows_outside_the_window():
     for tokens, cur in (([], 0), ([1] * 17, 0), ([1] * 8, 9), ([1], -1)):
         with pytest.raises(ValueError):
             tr.prefill(tokens, cur)
+
+
+@pytest.mark.parametrize("n", [8, 511, 513, 1100])
+def test_prompt_in_page_locked_memory_may_be_overwritten_after_the_call(n):
+    """The ids are read before nnb200_gpt_prefill returns, also from page-locked memory and behind work still queued."""
+    import ctypes as C
+    import torch
+    from tests import gpu_util as g
+    tr = _trainer(g.nnb, 72, 32, 1, 1, 64, 1104, 1, 1, 2, 0)
+    ids = np.random.default_rng(n).integers(0, 72, n).astype(np.int32)
+    want = tr.prefill(ids).clone()
+    buf = torch.from_numpy(ids.copy()).pin_memory()
+    busy = torch.randn(4096, 4096, device="cuda")
+    for _ in range(20):                                          # milliseconds of work in front of the call
+        busy = busy @ busy * 1e-3
+    ws, logits = tr._decode_state()
+    g.call("nnb200_gpt_prefill", C.byref(tr._c), g.ptr(tr.params), g.ptr(tr.shadow), g.ptr(ws), C.c_void_p(buf.data_ptr()), n, 0, g.ptr(logits), g.stream())
+    buf.fill_(1)
+    torch.cuda.synchronize()
+    assert torch.equal(logits, want)
