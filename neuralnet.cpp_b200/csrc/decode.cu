@@ -8,7 +8,9 @@
 // for the 12-layer benchmark model) but the chain of about sixty dependent kernels, each of which would wait for its
 // predecessor, then for its first loads.  So each is launched while its predecessor runs (programmatic dependent launch),
 // loads what does not depend on it - its first weights, the norm's scale, the cached keys and values - into registers,
-// and only then waits for it.  The normalisation before a projection is done while the input vector is staged in shared
+// and only then waits for it.  What the predecessor writes changes while the dependent kernel runs: such a pointer is not
+// `const __restrict__`, which would promise the compiler constant memory that it may read early, and through the
+// non-coherent path.  The normalisation before a projection is done while the input vector is staged in shared
 // memory (every block does it for itself: the vector is a few KB), the activation in fc1's epilogue, the rotation of Q
 // and K in the attention kernel.  Nothing may read, before its wait, what a kernel of the same token writes.
 // The token id, position and cache length are read from device memory, so that the launches of a token are the same
@@ -79,6 +81,20 @@ static int set_prompt(int* tok, const int* tokens_host, int n, cudaStream_t s)
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Loads of what the predecessor wrote: volatile, so that they stay behind the wait, and not held up by stores to shared memory.
+__device__ __forceinline__ float ld_produced(const float* p)
+{
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_produced4(const float* p)
+{
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
 template <typename... P, typename... A>
 static int launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem, int cluster, cudaStream_t s, A... args)
 {
@@ -119,9 +135,9 @@ __global__ void decode_embed_kernel(const float* __restrict__ tok_emb, const flo
 // R is 1 where there are too few rows for more than a warp each (latency), 4 for the LM head (12 us of bytes: fewer
 // stagings of x per row).
 template <typename WT, bool NORM, int R, int ACT>
-__global__ void __launch_bounds__(256, 3) gemv_kernel(const WT* __restrict__ W, const float* __restrict__ x, const float* __restrict__ gamma,
+__global__ void __launch_bounds__(256, 3) gemv_kernel(const WT* __restrict__ W, const float* x, const float* __restrict__ gamma,
                                                    const float* __restrict__ beta, int layer, const float* __restrict__ bias,
-                                                   const float* __restrict__ residual, float* __restrict__ y, int out, int in)
+                                                   const float* residual, float* __restrict__ y, int out, int in)
 {
     static_assert(ACT != 1 || R == 2, "SwiGLU takes a gate and an up row");
     constexpr int VN = Vec16<WT>::N, NC = 8 / R;
@@ -156,7 +172,7 @@ __global__ void __launch_bounds__(256, 3) gemv_kernel(const WT* __restrict__ W, 
     pdl_wait();
     if (in_regs) {
         const bool mine = t * 4 < in;
-        float4 v = mine ? *reinterpret_cast<const float4*>(x + t * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 v = mine ? ld_produced4(x + t * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (layer) {
             const float mean = block_sum((v.x + v.y) + (v.z + v.w), red) / static_cast<float>(in);
             if (mine) { v.x -= mean; v.y -= mean; v.z -= mean; v.w -= mean; }
@@ -166,10 +182,10 @@ __global__ void __launch_bounds__(256, 3) gemv_kernel(const WT* __restrict__ W, 
     } else {
         if ((in & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
 #pragma unroll 4
-            for (int c = t * 4; c < in; c += 1024) *reinterpret_cast<float4*>(xs + c) = *reinterpret_cast<const float4*>(x + c);
+            for (int c = t * 4; c < in; c += 1024) *reinterpret_cast<float4*>(xs + c) = ld_produced4(x + c);
         } else {
 #pragma unroll 4
-            for (int c = t; c < in; c += 256) xs[c] = x[c];
+            for (int c = t; c < in; c += 256) xs[c] = ld_produced(x + c);
         }
         if (NORM) {
             float mean = 0.f;
@@ -239,7 +255,7 @@ __global__ void __launch_bounds__(256, 3) gemv_kernel(const WT* __restrict__ W, 
                 if (!row_ok(u, r)) continue;
                 float v = acc[r] + bias[o];
                 if (ACT == 2) v = v / (1.0f + expf(-1.702f * v));
-                y[o] = v + (residual ? residual[o] : 0.f);
+                y[o] = v + (residual ? ld_produced(residual + o) : 0.f);
             }
         }
     }
@@ -254,7 +270,7 @@ __global__ void __launch_bounds__(256, 3) gemv_kernel(const WT* __restrict__ W, 
 // Bound by the chain wait - scores - merge.  (12 heads of 64 behind 900 tokens took 22.6 us when blocks of 32 rows left partial
 // results in global memory and the last one merged them; a whole layer, this kernel and four products, takes 17 us now.)
 template <int LPR, int NV, bool VEC>
-__global__ void __launch_bounds__(256) decode_attn_kernel(const float* __restrict__ qkv, float* __restrict__ kc, float* __restrict__ vc,
+__global__ void __launch_bounds__(256) decode_attn_kernel(const float* qkv, float* __restrict__ kc, float* __restrict__ vc,
                                                           float* __restrict__ out, const float* __restrict__ rope, const int* __restrict__ step,
                                                           int seq, int d, int dk, int heads, int alibi, float scale)
 {
