@@ -105,15 +105,28 @@ __device__ __forceinline__ bool tile_open(const ScoreMask& mk, int i0, int j0)
     return __syncthreads_or(any);
 }
 
+// A closed pair has weight 0, which takes it out of the sums as long as what it multiplies is finite.  So each block looks at
+// its results when it is done: one that is infinite or NaN may come of a closed pair, and the block starts again with the
+// guarded form, which adds open pairs only.  An infinite or NaN row thus reaches the positions that see it and no others,
+// whose results are the same bits either way.  (Looking at the staged rows of every tile instead cost 3 to 9 % of the forward.)
+template <int W> __device__ __forceinline__ bool not_finite(const float (&v)[4][W], int row0, int rows, int cols)
+{
+    bool bad = false;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < W; ++c) bad = bad || (row0 + r < rows && tile_col<W>(c) < cols && !isfinite(v[r][c]));
+    return bad;
+}
+
 // Queries are rows q0 .. S - 1 of a sequence of S keys (q0 = 0 in training; a prompt pass continues behind q0 cached rows), so
-// q and out point at the row of query q0; `lse` may be null.
-template <typename T, int DK>
-__global__ void __launch_bounds__(256) attn_fwd_simt_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ kc, const T* __restrict__ vc,
-                                                            long long ldk, T* __restrict__ out, float* __restrict__ lse, const int* __restrict__ doc,
-                                                            int B, int S, int q0, int H, int alibi, float scale)
+// q and out point at the row of query q0; `lse` may be null.  True, with nothing written: to be done again, guarded.
+template <typename T, int DK, bool GUARD>
+__device__ __forceinline__ bool attn_fwd_block(float* sm, const T* __restrict__ q, long long ldq, const T* __restrict__ kc, const T* __restrict__ vc,
+                                               long long ldk, T* __restrict__ out, float* __restrict__ lse, const int* __restrict__ doc,
+                                               int B, int S, int q0, int H, int alibi, float scale)
 {
     using D = SimtDims<DK>;
-    extern __shared__ __align__(16) float sm[];
     float *Qs = sm, *Ks = Qs + DK * kTilePitch, *Vs = Ks + DK * kTilePitch, *Ps = Vs + D::ROWS;
     const int nq = S - q0;
     const int bh = blockIdx.x % (B * H), qt = static_cast<int>(ceil_div(nq, kTile)) - 1 - blockIdx.x / (B * H), h = bh % H, b = bh / H;   // long rows first
@@ -160,8 +173,10 @@ __global__ void __launch_bounds__(256) attn_fwd_simt_kernel(const T* __restrict_
         }
         put_transposed(Ps, s);
         __syncthreads();
-        tile_rows_product<D::W, DK>(o, Ps, Vs);
+        if constexpr (GUARD) tile_rows_product<D::W, DK>(o, Ps, Vs, [&](int k, int r) { return mk.open(i0 + r, j0 + k); });
+        else tile_rows_product<D::W, DK>(o, Ps, Vs);
     }
+    if (!GUARD && __syncthreads_or(not_finite(o, i0 + ty * 4, S, DK))) return true;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int i = i0 + ty * 4 + r;
@@ -173,16 +188,31 @@ __global__ void __launch_bounds__(256) attn_fwd_simt_kernel(const T* __restrict_
             if (tile_col<D::W>(c) < DK) op[tile_col<D::W>(c)] = from_f32<T>(o[r][c] * inv);
         if (tx == 0 && lse) lse[(static_cast<size_t>(b) * H + h) * S + i] = m[r] + logf(l[r]);
     }
+    return false;
+}
+template <typename T, int DK>
+__device__ __noinline__ void attn_fwd_guarded(float* sm, const T* q, long long ldq, const T* kc, const T* vc, long long ldk, T* out, float* lse,
+                                              const int* doc, int B, int S, int q0, int H, int alibi, float scale)
+{
+    attn_fwd_block<T, DK, true>(sm, q, ldq, kc, vc, ldk, out, lse, doc, B, S, q0, H, alibi, scale);
+}
+template <typename T, int DK>
+__global__ void __launch_bounds__(256) attn_fwd_simt_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ kc, const T* __restrict__ vc,
+                                                            long long ldk, T* __restrict__ out, float* __restrict__ lse, const int* __restrict__ doc,
+                                                            int B, int S, int q0, int H, int alibi, float scale)
+{
+    extern __shared__ __align__(16) float sm[];
+    if (attn_fwd_block<T, DK, false>(sm, q, ldq, kc, vc, ldk, out, lse, doc, B, S, q0, H, alibi, scale))
+        attn_fwd_guarded<T, DK>(sm, q, ldq, kc, vc, ldk, out, lse, doc, B, S, q0, H, alibi, scale);
 }
 
 // dQ_i = scale sum_j P_ij (dP_ij - D_i) k_j
-template <typename T, int DK>
-__global__ void __launch_bounds__(256) attn_bwd_dq_simt_kernel(const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
-                                                               const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc,
-                                                               int B, int S, int H, int alibi, float scale)
+template <typename T, int DK, bool GUARD>
+__device__ __forceinline__ bool attn_bwd_dq_block(float* sm, const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
+                                                  const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc,
+                                                  int B, int S, int H, int alibi, float scale)
 {
     using D = SimtDims<DK>;
-    extern __shared__ __align__(16) float sm[];
     float *Qs = sm, *Gs = Qs + DK * kTilePitch, *Ks = Gs + DK * kTilePitch, *Vs = Ks + D::KC * kTilePitch, *Kr = Vs + D::KC * kTilePitch, *Ps = Kr + D::ROWS;
     const int bh = blockIdx.x % (B * H), qt = static_cast<int>(ceil_div(S, kTile)) - 1 - blockIdx.x / (B * H), h = bh % H, b = bh / H;
     const int d = H * DK, ld = 3 * d, i0 = qt * kTile, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -226,8 +256,10 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_simt_kernel(const T* __restri
         }
         put_transposed(Ps, s);
         __syncthreads();
-        tile_rows_product<D::W, DK>(dq, Ps, Kr);
+        if constexpr (GUARD) tile_rows_product<D::W, DK>(dq, Ps, Kr, [&](int k, int r) { return mk.open(i0 + r, j0 + k); });
+        else tile_rows_product<D::W, DK>(dq, Ps, Kr);
     }
+    if (!GUARD && __syncthreads_or(not_finite(dq, i0 + ty * 4, S, DK))) return true;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int i = i0 + ty * 4 + r;
@@ -237,16 +269,31 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_simt_kernel(const T* __restri
         for (int c = 0; c < D::W; ++c)
             if (tile_col<D::W>(c) < DK) p[tile_col<D::W>(c)] = from_f32<T>(scale * dq[r][c]);
     }
+    return false;
+}
+template <typename T, int DK>
+__device__ __noinline__ void attn_bwd_dq_guarded(float* sm, const T* qkv, const T* dout, const float* lse, const float* dvec, T* dqkv, const int* doc,
+                                                 int B, int S, int H, int alibi, float scale)
+{
+    attn_bwd_dq_block<T, DK, true>(sm, qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale);
+}
+template <typename T, int DK>
+__global__ void __launch_bounds__(256) attn_bwd_dq_simt_kernel(const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
+                                                               const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc,
+                                                               int B, int S, int H, int alibi, float scale)
+{
+    extern __shared__ __align__(16) float sm[];
+    if (attn_bwd_dq_block<T, DK, false>(sm, qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale))
+        attn_bwd_dq_guarded<T, DK>(sm, qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale);
 }
 
 // dK_j = scale sum_i P_ij (dP_ij - D_i) q_i ; dV_j = sum_i P_ij dO_i.  Rows of the tile are keys, columns queries.
-template <typename T, int DK>
-__global__ void __launch_bounds__(256) attn_bwd_dkv_simt_kernel(const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
-                                                                const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc,
-                                                                int B, int S, int H, int alibi, float scale)
+template <typename T, int DK, bool GUARD>
+__device__ __forceinline__ bool attn_bwd_dkv_block(float* sm, const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
+                                                   const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc,
+                                                   int B, int S, int H, int alibi, float scale)
 {
     using D = SimtDims<DK>;
-    extern __shared__ __align__(16) float sm[];
     float *Ks = sm, *Vs = Ks + D::KC * kTilePitch, *Qs = Vs + D::KC * kTilePitch, *Gs = Qs + D::KC * kTilePitch, *Qr = Gs + D::KC * kTilePitch,
           *Gr = Qr + D::ROWS, *Ps = Gr + D::ROWS, *Ss = Ps + kTileFloats;
     const int bh = blockIdx.x % (B * H), kt = blockIdx.x / (B * H), h = bh % H, b = bh / H;      // the first keys are seen by the most queries
@@ -291,9 +338,16 @@ __global__ void __launch_bounds__(256) attn_bwd_dkv_simt_kernel(const T* __restr
         put_transposed(Ps, s);
         put_transposed(Ss, dp);
         __syncthreads();
-        tile_rows_product<D::W, DK>(dv, Ps, Gr);
-        tile_rows_product<D::W, DK>(dk, Ss, Qr);
+        if constexpr (GUARD) {
+            auto open = [&](int k, int r) { return mk.open(i0 + k, j0 + r); };
+            tile_rows_product<D::W, DK>(dv, Ps, Gr, open);
+            tile_rows_product<D::W, DK>(dk, Ss, Qr, open);
+        } else {
+            tile_rows_product<D::W, DK>(dv, Ps, Gr);
+            tile_rows_product<D::W, DK>(dk, Ss, Qr);
+        }
     }
+    if (!GUARD && __syncthreads_or(not_finite(dk, j0 + ty * 4, S, DK) || not_finite(dv, j0 + ty * 4, S, DK))) return true;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const int j = j0 + ty * 4 + r;
@@ -305,6 +359,22 @@ __global__ void __launch_bounds__(256) attn_bwd_dkv_simt_kernel(const T* __restr
             if (col < DK) { p[col] = from_f32<T>(scale * dk[r][c]); p[d + col] = from_f32<T>(dv[r][c]); }
         }
     }
+    return false;
+}
+template <typename T, int DK>
+__device__ __noinline__ void attn_bwd_dkv_guarded(float* sm, const T* qkv, const T* dout, const float* lse, const float* dvec, T* dqkv, const int* doc,
+                                                  int B, int S, int H, int alibi, float scale)
+{
+    attn_bwd_dkv_block<T, DK, true>(sm, qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale);
+}
+template <typename T, int DK>
+__global__ void __launch_bounds__(256) attn_bwd_dkv_simt_kernel(const T* __restrict__ qkv, const T* __restrict__ dout, const float* __restrict__ lse,
+                                                                const float* __restrict__ dvec, T* __restrict__ dqkv, const int* __restrict__ doc,
+                                                                int B, int S, int H, int alibi, float scale)
+{
+    extern __shared__ __align__(16) float sm[];
+    if (attn_bwd_dkv_block<T, DK, false>(sm, qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale))
+        attn_bwd_dkv_guarded<T, DK>(sm, qkv, dout, lse, dvec, dqkv, doc, B, S, H, alibi, scale);
 }
 
 template <int DK> constexpr int simt_smem_fwd() { return (2 * DK * kTilePitch + SimtDims<DK>::ROWS + kTileFloats) * 4; }

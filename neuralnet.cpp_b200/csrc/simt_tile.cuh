@@ -79,9 +79,11 @@ __device__ __forceinline__ void tile_product(float (&acc)[4][4], const float* __
     for (int r = 0; r < 4; ++r) { unpack2(s[r][0], acc[r][0], acc[r][1]); unpack2(s[r][1], acc[r][2], acc[r][3]); }
 }
 
-// acc[r][c] += sum_{k < 64} A[k][4 ty + r] * B[k][W tx + c], rows of B of `pitch` floats; threads with W tx >= C have nothing
-template <int W, int C>
-__device__ __forceinline__ void tile_rows_product(float (&acc)[4][W], const float* __restrict__ A, const float* __restrict__ B)
+// acc[r][c] += sum_{k < 64} A[k][4 ty + r] * B[k][W tx + c] over the terms with open(k, 4 ty + r), rows of B of C + 4 floats;
+// threads with W tx >= C have nothing
+struct AllOpen { __device__ __forceinline__ bool operator()(int, int) const { return true; } };
+template <int W, int C, typename Open = AllOpen>
+__device__ __forceinline__ void tile_rows_product(float (&acc)[4][W], const float* __restrict__ A, const float* __restrict__ B, Open open = {})
 {
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     if (W * tx >= C) return;
@@ -102,9 +104,11 @@ __device__ __forceinline__ void tile_rows_product(float (&acc)[4][W], const floa
             for (int c = 0; c < W; ++c) b[c] = B[k * (C + 4) + W * tx + c];
         }
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < 4; ++r) {
+            if (!open(k, ty * 4 + r)) continue;
 #pragma unroll
             for (int c = 0; c < W; ++c) acc[r][c] = fmaf(av[r], b[c], acc[r][c]);
+        }
     }
 }
 // column of accumulator entry c of tile_rows_product

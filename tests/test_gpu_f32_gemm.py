@@ -87,3 +87,58 @@ def test_attention_f32_tile_edges(g, dk, S, docs):
     # fp32 sums of up to 200 terms and an exponential of arguments up to about 50 (error 50 x 2^-24): 1e-5 of the norm
     assert (out - ref).norm() <= 1e-5 * ref.norm()
     assert (dqkv - x.grad).norm() <= 1e-5 * x.grad.norm()
+
+
+def _attention(g, qkv, dout, doc, B, S, H, dk, precision):
+    import torch
+    out, lse, dqkv, dvec = torch.empty_like(dout), torch.empty(B * H * S, device="cuda"), torch.empty_like(qkv), torch.empty(B * H * S, device="cuda")
+    g.call("nnb200_attention_forward", g.ptr(qkv), g.ptr(out), g.ptr(lse), g.ptr(doc), None, B, S, H, dk, 0, precision, g.stream())
+    g.call("nnb200_attention_backward", g.ptr(qkv), g.ptr(out), g.ptr(dout), g.ptr(lse), g.ptr(dvec), g.ptr(dqkv), g.ptr(doc), None, B, S, H, dk, 0, precision,
+           g.stream())
+    torch.cuda.synchronize()
+    return [t.float().view(B, S, -1, H * dk) for t in (out, dqkv)]
+
+
+# fp32 at every head size, and the bf16 forms that run the same kernels (small heads, heads of 128 at a ragged length)
+@pytest.mark.parametrize("dk,precision", [(8, 0), (32, 0), (64, 0), (128, 0), (8, 1), (16, 1), (128, 1)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_attention_keeps_non_finite_rows_from_queries_that_do_not_see_them(g, dk, precision, value):
+    """An infinite or NaN row reaches the positions that attend to it (or that it attends to, in the gradients of keys and
+    values) and leaves every other result bit for bit what it is without that row."""
+    import torch
+    B, H, S, at = 1, 2, 200, 100                                 # `at` in the middle of a 64-row tile
+    d = H * dk
+    dt = torch.bfloat16 if precision else torch.float32
+    gen = torch.Generator(device="cuda").manual_seed(dk)
+    qkv = torch.randn(B * S, 3 * d, device="cuda", generator=gen).to(dt)
+    dout = torch.randn(B * S, d, device="cuda", generator=gen).to(dt)
+    out, dqkv = _attention(g, qkv, dout, None, B, S, H, dk, precision)
+    for part in range(4):                                        # a row of q, k, v or dout
+        x, y = qkv.clone(), dout.clone()
+        if part < 3:
+            x[at, part * d:(part + 1) * d] = value
+        else:
+            y[at] = value
+        o, dx = _attention(g, x, y, None, B, S, H, dk, precision)
+        before, after = slice(0, at), slice(at + 1, S)
+        if part == 3:                                            # no output depends on it
+            assert torch.equal(o, out)
+        elif part == 0:                                          # its own output
+            assert not torch.isfinite(o[:, at]).any()
+            assert torch.equal(o[:, before], out[:, before]) and torch.equal(o[:, after], out[:, after])
+        else:                                                    # a key or value: the queries from there on
+            assert torch.equal(o[:, before], out[:, before])
+            if part == 2 or value != value:                      # (an infinite key may score minus infinity)
+                assert not torch.isfinite(o[:, after]).any()
+        assert torch.equal(dx[:, before, 0], dqkv[:, before, 0])               # dQ of earlier queries
+        if part in (0, 3):                                       # a query's row: no later query, no later key or value
+            assert torch.equal(dx[:, after], dqkv[:, after])
+            assert not torch.isfinite(dx[:, at, 0]).any() and not torch.isfinite(dx[:, before, 1]).any()
+    # one document in which every row of everything is broken, between documents that are whole
+    doc = (torch.arange(S, device="cuda") // 50).to(torch.int32).contiguous()
+    out, dqkv = _attention(g, qkv, dout, doc, B, S, H, dk, precision)
+    x, y = qkv.clone(), dout.clone()
+    x[50:100], y[50:100] = value, value
+    o, dx = _attention(g, x, y, doc, B, S, H, dk, precision)
+    whole = torch.cat([torch.arange(50), torch.arange(100, S)]).cuda()
+    assert torch.equal(o[:, whole], out[:, whole]) and torch.equal(dx[:, whole], dqkv[:, whole])
