@@ -82,6 +82,11 @@ static int launch_dvec(const T* out, const T* dout, float* dvec, int B, int S, i
 // What bounds them: the fp32 pipe at long sequences; at short ones (few blocks) the chain stage - product - exponential.
 // 8 x 128 x 4 heads of 32, fp32: forward 15 us, dQ 14, dK / dV 18 (with one warp per row and lanes over the keys, whose loads
 // were a row length apart: 123, 132, 179).
+// Terms of a run in the sums over keys and queries (tile_rows_product).  Errors of out, dQ, dK, dV against float64, 2048 queries
+// and keys, heads of 64 (units of 1e-7): runs of 8: 2.5, 3.8, 4.0, 3.4; one chain: 4.0, 5.2, 10.8, 11.1; a warp per row with its
+// lanes over the other index: 2.4, 3.7, 4.1, 3.6.  8 x 512 x 6 heads of 64, gradients: 304 us as one chain, 315 in runs.
+// bf16 results are rounded a thousand times coarser: one chain.
+template <typename T> constexpr int kRun = sizeof(T) == 4 ? 8 : kTile;
 template <int DK> struct SimtDims {
     static constexpr int KC = DK < 64 ? DK : 64, W = tile_width(DK), ROWS = kTile * (DK + 4);
 };
@@ -173,8 +178,8 @@ __device__ __forceinline__ bool attn_fwd_block(float* sm, const T* __restrict__ 
         }
         put_transposed(Ps, s);
         __syncthreads();
-        if constexpr (GUARD) tile_rows_product<D::W, DK>(o, Ps, Vs, [&](int k, int r) { return mk.open(i0 + r, j0 + k); });
-        else tile_rows_product<D::W, DK>(o, Ps, Vs);
+        if constexpr (GUARD) tile_rows_product<D::W, DK, kRun<T>>(o, Ps, Vs, [&](int k, int r) { return mk.open(i0 + r, j0 + k); });
+        else tile_rows_product<D::W, DK, kRun<T>>(o, Ps, Vs);
     }
     if (!GUARD && __syncthreads_or(not_finite(o, i0 + ty * 4, S, DK))) return true;
 #pragma unroll
@@ -256,8 +261,8 @@ __device__ __forceinline__ bool attn_bwd_dq_block(float* sm, const T* __restrict
         }
         put_transposed(Ps, s);
         __syncthreads();
-        if constexpr (GUARD) tile_rows_product<D::W, DK>(dq, Ps, Kr, [&](int k, int r) { return mk.open(i0 + r, j0 + k); });
-        else tile_rows_product<D::W, DK>(dq, Ps, Kr);
+        if constexpr (GUARD) tile_rows_product<D::W, DK, kRun<T>>(dq, Ps, Kr, [&](int k, int r) { return mk.open(i0 + r, j0 + k); });
+        else tile_rows_product<D::W, DK, kRun<T>>(dq, Ps, Kr);
     }
     if (!GUARD && __syncthreads_or(not_finite(dq, i0 + ty * 4, S, DK))) return true;
 #pragma unroll
@@ -340,11 +345,11 @@ __device__ __forceinline__ bool attn_bwd_dkv_block(float* sm, const T* __restric
         __syncthreads();
         if constexpr (GUARD) {
             auto open = [&](int k, int r) { return mk.open(i0 + k, j0 + r); };
-            tile_rows_product<D::W, DK>(dv, Ps, Gr, open);
-            tile_rows_product<D::W, DK>(dk, Ss, Qr, open);
+            tile_rows_product<D::W, DK, kRun<T>>(dv, Ps, Gr, open);
+            tile_rows_product<D::W, DK, kRun<T>>(dk, Ss, Qr, open);
         } else {
-            tile_rows_product<D::W, DK>(dv, Ps, Gr);
-            tile_rows_product<D::W, DK>(dk, Ss, Qr);
+            tile_rows_product<D::W, DK, kRun<T>>(dv, Ps, Gr);
+            tile_rows_product<D::W, DK, kRun<T>>(dk, Ss, Qr);
         }
     }
     if (!GUARD && __syncthreads_or(not_finite(dk, j0 + ty * 4, S, DK) || not_finite(dv, j0 + ty * 4, S, DK))) return true;

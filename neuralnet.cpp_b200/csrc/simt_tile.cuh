@@ -80,35 +80,56 @@ __device__ __forceinline__ void tile_product(float (&acc)[4][4], const float* __
 }
 
 // acc[r][c] += sum_{k < 64} A[k][4 ty + r] * B[k][W tx + c] over the terms with open(k, 4 ty + r), rows of B of C + 4 floats;
-// threads with W tx >= C have nothing
+// threads with W tx >= C have nothing.  The terms are added up in runs of RUN, the runs of a tile with one another, and the
+// tile to acc: one chain over all rows rounds at its full size every time, an error that grows with their number.
 struct AllOpen { __device__ __forceinline__ bool operator()(int, int) const { return true; } };
-template <int W, int C, typename Open = AllOpen>
+template <int W, int C, int RUN = kTile, typename Open = AllOpen>
 __device__ __forceinline__ void tile_rows_product(float (&acc)[4][W], const float* __restrict__ A, const float* __restrict__ B, Open open = {})
 {
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     if (W * tx >= C) return;
+    auto add_terms = [&](float (&to)[4][W], int k0) {
 #pragma unroll 4
-    for (int k = 0; k < kTile; ++k) {
-        const float4 a = *reinterpret_cast<const float4*>(A + k * kTilePitch + ty * 4);
-        const float av[4] = {a.x, a.y, a.z, a.w};
-        float b[W];
-        // W >= 4: columns 4 tx .. of each run of 64, so that a warp's vectors are contiguous
-        if constexpr (W >= 4) {
+        for (int k = k0; k < k0 + RUN; ++k) {
+            const float4 a = *reinterpret_cast<const float4*>(A + k * kTilePitch + ty * 4);
+            const float av[4] = {a.x, a.y, a.z, a.w};
+            float b[W];
+            // W >= 4: columns 4 tx .. of each run of 64, so that a warp's vectors are contiguous
+            if constexpr (W >= 4) {
 #pragma unroll
-            for (int g = 0; g < W / 4; ++g) {
-                const float4 x = *reinterpret_cast<const float4*>(B + k * (C + 4) + g * 64 + tx * 4);
-                b[4 * g] = x.x; b[4 * g + 1] = x.y; b[4 * g + 2] = x.z; b[4 * g + 3] = x.w;
+                for (int g = 0; g < W / 4; ++g) {
+                    const float4 x = *reinterpret_cast<const float4*>(B + k * (C + 4) + g * 64 + tx * 4);
+                    b[4 * g] = x.x; b[4 * g + 1] = x.y; b[4 * g + 2] = x.z; b[4 * g + 3] = x.w;
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < W; ++c) b[c] = B[k * (C + 4) + W * tx + c];
             }
-        } else {
 #pragma unroll
-            for (int c = 0; c < W; ++c) b[c] = B[k * (C + 4) + W * tx + c];
+            for (int r = 0; r < 4; ++r) {
+                if (!open(k, ty * 4 + r)) continue;
+#pragma unroll
+                for (int c = 0; c < W; ++c) to[r][c] = fmaf(av[r], b[c], to[r][c]);
+            }
+        }
+    };
+    if constexpr (RUN == kTile) {
+        add_terms(acc, 0);
+    } else {
+        float tile[4][W] = {};
+#pragma unroll 1
+        for (int k0 = 0; k0 < kTile; k0 += RUN) {
+            float part[4][W] = {};
+            add_terms(part, k0);
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < W; ++c) tile[r][c] += part[r][c];
         }
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            if (!open(k, ty * 4 + r)) continue;
+        for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int c = 0; c < W; ++c) acc[r][c] = fmaf(av[r], b[c], acc[r][c]);
-        }
+            for (int c = 0; c < W; ++c) acc[r][c] += tile[r][c];
     }
 }
 // column of accumulator entry c of tile_rows_product

@@ -142,3 +142,26 @@ def test_attention_keeps_non_finite_rows_from_queries_that_do_not_see_them(g, dk
     o, dx = _attention(g, x, y, doc, B, S, H, dk, precision)
     whole = torch.cat([torch.arange(50), torch.arange(100, S)]).cuda()
     assert torch.equal(o[:, whole], out[:, whole]) and torch.equal(dx[:, whole], dqkv[:, whole])
+
+
+@pytest.mark.parametrize("dk", [16, 64])
+def test_attention_loses_no_precision_with_the_length_of_the_sequence(g, dk):
+    """Every output adds a term per key or query.  In one chain over 2048 of them the error is sqrt(2048 / 64) = 5.7 times that
+    over 64 (2.8 to 5 measured, with what the terms bring along); in runs of 8, tiles of 8 runs and a chain over tiles it goes
+    with 8 + 8 + n / 64: sqrt(48 / 17) = 1.7 times."""
+    import torch
+    err = []
+    for S in (64, 2048):
+        B, H = 2048 // S, 2
+        d = H * dk
+        gen = torch.Generator(device="cuda").manual_seed(dk)
+        qkv, dout = torch.randn(B * S, 3 * d, device="cuda", generator=gen), torch.randn(B * S, d, device="cuda", generator=gen)
+        out, dqkv = (t.double().reshape(B * S, -1) for t in _attention(g, qkv, dout, None, B, S, H, dk, 0))
+        x = qkv.double().requires_grad_()
+        q, k, v = x.view(B, S, 3, H, dk).permute(2, 0, 3, 1, 4)
+        s = (q @ k.transpose(-1, -2) / dk ** 0.5).masked_fill(torch.ones(S, S, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+        ref = (s.softmax(-1) @ v).transpose(1, 2).reshape(B * S, d)
+        ref.backward(dout.double())
+        pairs = [(out, ref.detach())] + [(dqkv[:, c * d:(c + 1) * d], x.grad[:, c * d:(c + 1) * d]) for c in range(3)]
+        err.append([float((a - b).norm() / b.norm()) for a, b in pairs])
+    assert all(long < 1.8 * short for short, long in zip(*err)), err
