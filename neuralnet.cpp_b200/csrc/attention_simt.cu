@@ -84,7 +84,7 @@ static int launch_dvec(const T* out, const T* dout, float* dvec, int B, int S, i
 // were a row length apart: 123, 132, 179).
 // Terms of a run in the sums over keys and queries (tile_rows_product).  Errors of out, dQ, dK, dV against float64, 2048 queries
 // and keys, heads of 64 (units of 1e-7): runs of 8: 2.5, 3.8, 4.0, 3.4; one chain: 4.0, 5.2, 10.8, 11.1; a warp per row with its
-// lanes over the other index: 2.4, 3.7, 4.1, 3.6.  8 x 512 x 6 heads of 64, gradients: 304 us as one chain, 315 in runs.
+// lanes over the other index: 2.4, 3.7, 4.1, 3.6.  8 x 512 x 6 heads of 64, gradients: 304 us as one chain, 303 in runs.
 // bf16 results are rounded a thousand times coarser: one chain.
 template <typename T> constexpr int kRun = sizeof(T) == 4 ? 8 : kTile;
 template <int DK> struct SimtDims {

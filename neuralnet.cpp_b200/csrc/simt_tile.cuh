@@ -89,7 +89,7 @@ __device__ __forceinline__ void tile_rows_product(float (&acc)[4][W], const floa
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     if (W * tx >= C) return;
     auto add_terms = [&](float (&to)[4][W], int k0) {
-#pragma unroll 4
+#pragma unroll(RUN < 8 ? RUN : RUN == kTile ? 4 : 8)
         for (int k = k0; k < k0 + RUN; ++k) {
             const float4 a = *reinterpret_cast<const float4*>(A + k * kTilePitch + ty * 4);
             const float av[4] = {a.x, a.y, a.z, a.w};
