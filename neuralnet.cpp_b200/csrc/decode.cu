@@ -269,14 +269,18 @@ __global__ void __launch_bounds__(256, 3) gemv_kernel(const WT* __restrict__ W, 
 // fixed order.  The grid is the same for every cache length.
 // Bound by the chain wait - scores - merge.  (12 heads of 64 behind 900 tokens took 22.6 us when blocks of 32 rows left partial
 // results in global memory and the last one merged them; a whole layer, this kernel and four products, takes 17 us now.)
-template <int LPR, int NV, bool VEC>
-__global__ void __launch_bounds__(256) decode_attn_kernel(const float* qkv, float* __restrict__ kc, float* __restrict__ vc,
+// Behind long contexts by the latency of a round of rows: where a row takes a whole warp, blocks have 512 threads and load the
+// next round's rows as soon as this round's were used (a step of two layers, one head of 128 behind 65535 rows: 372 us; 1366
+// with the loads at the start of a round and 256 threads, 780 with blocks of 32 rows).
+template <int LPR, int NV, bool VEC, int THREADS>
+__global__ void __launch_bounds__(THREADS) decode_attn_kernel(const float* qkv, float* __restrict__ kc, float* __restrict__ vc,
                                                           float* __restrict__ out, const float* __restrict__ rope, const int* __restrict__ step,
                                                           int seq, int d, int dk, int heads, int alibi, float scale)
 {
-    constexpr int B = 8 / NV, G = 256 / LPR, RANKS = 8, DMAX = LPR * NV * 4;
-    __shared__ float wm[8], wl[8];
-    __shared__ __align__(16) float wo[8][DMAX];
+    constexpr int B = 8 / NV, G = THREADS / LPR, RANKS = 8, DMAX = LPR * NV * 4, WARPS = THREADS / 32, ROUND = B * RANKS * G;
+    constexpr bool EARLY = THREADS == 512;                       // next round's keys and values loaded as soon as this round's were used
+    __shared__ float wm[WARPS], wl[WARPS];
+    __shared__ __align__(16) float wo[WARPS][DMAX];
     __shared__ float part[DMAX + 2];                            // this block's maximum, sum and weighted values
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, sub = t % LPR, h = blockIdx.x / RANKS;
     const int rank = static_cast<int>(cluster_ctarank()), g0 = rank * G + t / LPR;
@@ -296,17 +300,17 @@ __global__ void __launch_bounds__(256) decode_attn_kernel(const float* qkv, floa
         }
     };
     float kr[B][NV * 4], vr[B][NV * 4];
-    auto load = [&](int j0) {
+    auto load = [&](int j0, bool keys, bool values) {
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             const int j = j0 + b * (RANKS * G);
             if (j < cur) {
-                fetch(kc + static_cast<size_t>(j) * d + head, kr[b]);
-                fetch(vc + static_cast<size_t>(j) * d + head, vr[b]);
+                if (keys) fetch(kc + static_cast<size_t>(j) * d + head, kr[b]);
+                if (values) fetch(vc + static_cast<size_t>(j) * d + head, vr[b]);
             }
         }
     };
-    load(g0);
+    load(g0, true, true);
     pdl_launch();
     pdl_wait();
     // q or the new k: rotated with rotary positions by the cache row it lands in (table: cos (seq, dk/2), then sin)
@@ -328,8 +332,8 @@ __global__ void __launch_bounds__(256) decode_attn_kernel(const float* qkv, floa
     for (int i = 0; i < NV * 4; ++i) o[i] = 0.f;
     const float slope = alibi ? exp2f(-8.0f * static_cast<float>(h) / static_cast<float>(heads)) : 0.f;
     float m = -INFINITY, l = 0.f;
-    for (int j0 = g0; j0 - t / LPR % (32 / LPR) < n; j0 += B * RANKS * G) {     // the same number of rounds for all groups of a warp
-        if (j0 != g0) load(j0);
+    for (int j0 = g0; j0 - t / LPR % (32 / LPR) < n; j0 += ROUND) {             // the same number of rounds for all groups of a warp
+        if (!EARLY && j0 != g0) load(j0, true, true);
         float s[B];
         float mx = m;
 #pragma unroll
@@ -357,6 +361,7 @@ __global__ void __launch_bounds__(256) decode_attn_kernel(const float* qkv, floa
             s[b] = j < n ? a * scale - slope * static_cast<float>(cur - j) : -INFINITY;
             mx = fmaxf(mx, s[b]);
         }
+        if (EARLY) load(j0 + ROUND, true, false);
         const float ref = mx == -INFINITY ? 0.f : mx, back = expf(m - ref);
         m = mx;
         l *= back;
@@ -370,6 +375,7 @@ __global__ void __launch_bounds__(256) decode_attn_kernel(const float* qkv, floa
 #pragma unroll
             for (int i = 0; i < NV * 4; ++i) o[i] = fmaf(e, vr[b][i], o[i]);
         }
+        if (EARLY) load(j0 + ROUND, false, true);
     }
 #pragma unroll
     for (int w = LPR; w < 32; w <<= 1) {                        // groups of a warp
@@ -389,12 +395,12 @@ __global__ void __launch_bounds__(256) decode_attn_kernel(const float* qkv, floa
     {                                                           // warps of the block
         float bm = wm[0];
 #pragma unroll
-        for (int w = 1; w < 8; ++w) bm = fmaxf(bm, wm[w]);
+        for (int w = 1; w < WARPS; ++w) bm = fmaxf(bm, wm[w]);
         const float ref = bm == -INFINITY ? 0.f : bm;
         if (t < DMAX) {
             float bl = 0.f, a = 0.f;
 #pragma unroll
-            for (int w = 0; w < 8; ++w) { const float e = expf(wm[w] - ref); bl += wl[w] * e; a = fmaf(wo[w][t], e, a); }
+            for (int w = 0; w < WARPS; ++w) { const float e = expf(wm[w] - ref); bl += wl[w] * e; a = fmaf(wo[w][t], e, a); }
             part[2 + t] = a;
             if (t == 0) { part[0] = bm; part[1] = bl; }
         }
@@ -435,18 +441,22 @@ static int decode_attention(const float* qkv, float* kc, float* vc, float* out, 
 {
     const int d = c.d_model, dk = d / c.heads;
     const dim3 grid(static_cast<unsigned>(c.heads) * 8);
-    auto go = [&](auto* kernel) {
-        return launch_dependent(kernel, grid, 256, 0, 8, s, qkv, kc, vc, out, rope, step, c.seq, d, dk, c.heads, c.pos == 2 ? 1 : 0,
+    auto go = [&](auto* kernel, int threads) {
+        return launch_dependent(kernel, grid, threads, 0, 8, s, qkv, kc, vc, out, rope, step, c.seq, d, dk, c.heads, c.pos == 2 ? 1 : 0,
                                 1.0f / sqrtf(static_cast<float>(dk)));
     };
-    if (dk % 4 == 0 && ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0) {
-        if (dk <= 32) return go(decode_attn_kernel<8, 1, true>);
-        if (dk <= 64) return go(decode_attn_kernel<16, 1, true>);
-        if (dk <= 128) return go(decode_attn_kernel<32, 1, true>);
-        return go(decode_attn_kernel<32, 2, true>);
+    const bool vec = dk % 4 == 0 && ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15) == 0;
+    if (vec && dk <= 32) return go(decode_attn_kernel<8, 1, true, 256>, 256);
+    if (vec && dk <= 64) return go(decode_attn_kernel<16, 1, true, 256>, 256);
+    // A row that takes a whole warp leaves a cluster of 256 threads 64 rows at a time: 512 threads halve the rounds, as long as
+    // the blocks, which then fill an SM's registers, leave SMs free for the predecessor's (a step of two layers, heads of 128
+    // behind 900 | 8191 rows: 8 heads 43 | 212 us with 256 threads, 38 | 88 with 512; 16 heads 88 | 252 and 91 | 173).
+    if (c.heads <= 8) {
+        if (dk <= 128) return vec ? go(decode_attn_kernel<32, 1, true, 512>, 512) : go(decode_attn_kernel<32, 1, false, 512>, 512);
+        return vec ? go(decode_attn_kernel<32, 2, true, 512>, 512) : go(decode_attn_kernel<32, 2, false, 512>, 512);
     }
-    if (dk <= 128) return go(decode_attn_kernel<32, 1, false>);
-    return go(decode_attn_kernel<32, 2, false>);
+    if (dk <= 128) return vec ? go(decode_attn_kernel<32, 1, true, 256>, 256) : go(decode_attn_kernel<32, 1, false, 256>, 256);
+    return vec ? go(decode_attn_kernel<32, 2, true, 256>, 256) : go(decode_attn_kernel<32, 2, false, 256>, 256);
 }
 
 // `step` (device): token id, position, cache length

@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 # (heads, head size, d_ff, vocabulary, tokens)
 SHAPES = [(2, 6, 20, 33, 20), (1, 30, 36, 40, 9), (4, 24, 96, 64, 300), (2, 64, 2100, 72, 40), (9, 128, 64, 50, 12), (1, 128, 64, 64, 530), (1, 160, 72, 64, 270),
-          (3, 32, 100, 4097, 3)]
+          (3, 32, 100, 4097, 3),
+          # several rounds of the cluster: 1024 rows at 512 threads and one vector a lane, 512 at 256 threads or two vectors, 1024 of 64
+          (1, 128, 64, 64, 2100), (9, 128, 64, 50, 1100), (1, 160, 72, 64, 1100), (1, 66, 40, 64, 2100), (1, 64, 64, 64, 2100)]
 
 
 @pytest.mark.parametrize("heads,dk,ff,vocab,n", SHAPES)
