@@ -98,13 +98,16 @@ __global__ void __launch_bounds__(256) bmm_reduce_kernel(const float* __restrict
         score_tile<KC>(s, X, Y, i0, j0, d.K, Xs, Ys, keep);
         keep = 1;
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < 4; ++r) {
+            float part = init;                                    // of the tile: a chain over all tiles has one addition for each
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 if (mv[r][c] == -INFINITY) continue;              // masked entries: skipped for Sum and Min, no effect on Max
                 const float v = d.alpha * s[r][c] + mv[r][c];
-                acc[r] = DENOM ? acc[r] + expf(v - mx[r]) : combine(op, acc[r], v);
+                part = DENOM ? part + expf(v - mx[r]) : combine(op, part, v);
             }
+            acc[r] = combine(DENOM ? 0 : op, acc[r], part);
+        }
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
@@ -209,9 +212,12 @@ __global__ void __launch_bounds__(256) bmm_backward_q_kernel(const float* __rest
         score_tile<KC>(s, X, Y, i0, j0, d.K, Xs, Ys, keep);
         keep = 1;
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < 4; ++r) {
+            float part = 0.f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) R[r] += softmax_weight(s[r][c], mv[r][c], d.alpha, mx[r], inv_l[r]) * pv[r][c];
+            for (int c = 0; c < 4; ++c) part += softmax_weight(s[r][c], mv[r][c], d.alpha, mx[r], inv_l[r]) * pv[r][c];
+            R[r] += part;
+        }
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
