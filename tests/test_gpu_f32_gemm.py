@@ -165,3 +165,53 @@ def test_attention_loses_no_precision_with_the_length_of_the_sequence(g, dk):
         pairs = [(out, ref.detach())] + [(dqkv[:, c * d:(c + 1) * d], x.grad[:, c * d:(c + 1) * d]) for c in range(3)]
         err.append([float((a - b).norm() / b.norm()) for a, b in pairs])
     assert all(long < 1.8 * short for short, long in zip(*err)), err
+
+
+# persistent and split forms (K over 2, 4, 8 CTAs), tiles of 64 and 128 columns, edges in M, N and K
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(130, 70, 65), (300, 150, 200), (100, 60, 1000), (384, 128, 1024), (805, 377, 697), (3000, 2600, 70)])
+def test_gemm_f32_tiles_with_non_finite_results(g, M, N, K, a_mn, b_mn):
+    """Rows and columns with infinities and NaNs, or that overflow in bf16 or in the sum, next to finite ones in the same tiles."""
+    r = np.random.default_rng(M + N)
+    A, B = r.standard_normal((M, K)).astype(np.float32), r.standard_normal((N, K)).astype(np.float32)
+    rows, cols = r.choice(M, 6, replace=False), r.choice(N, 3, replace=False)
+    A[rows[0], K // 2], A[rows[1], 0], A[rows[2], K - 1] = np.inf, -np.inf, np.nan
+    B[cols[0], K // 3], B[cols[1], 1] = np.nan, np.inf
+    A[rows[3], 0], B[:, 0] = 3.4e38, np.abs(B[:, 0]) * 1e-30         # beyond bf16, results of 1e8
+    A[rows[4]] = np.abs(A[rows[4]]) * 3e37                           # infinite where a column adds up to more than about ten
+    c0 = r.standard_normal((M, N)).astype(np.float32)
+    a, b, c = g.dev(A.T if a_mn else A), g.dev(B.T if b_mn else B), g.dev(c0)
+    g.call("nnb200_gemm_f32", g.ptr(a), g.ptr(b), g.ptr(c), M, N, K, M if a_mn else K, N if b_mn else K, N, a_mn, b_mn, C.c_float(2.0), None, None, 1,
+           g.stream())
+    got = g.host(c)
+    with np.errstate(all="ignore"):
+        A64, B64 = A.astype(np.float64), B.astype(np.float64)
+        dot = A64 @ B64.T
+        scale = np.abs(A64) @ np.abs(B64).T
+    fine = np.isfinite(scale) & (scale < 1e38)                       # no fp32 sum overflows whatever its order
+    want = 2.0 * dot + c0
+    # one FMA chain over K where a result was computed again, else far less
+    assert (np.abs(got[fine] - want[fine]) <= (2.0 * scale * K * 2.0 ** -24 + 2.0 ** -22 * (np.abs(want) + np.abs(c0) + 1))[fine]).all()
+    special = ~np.isfinite(dot)
+    assert np.array_equal(np.isnan(got[special]), np.isnan(dot[special])) and np.array_equal(np.isposinf(got[special]), np.isposinf(dot[special]))
+    assert g.gemm_status() == 0
+
+
+def test_gemm_f32_full_of_nans_is_not_slow(g):
+    """A diverged run multiplies matrices full of NaNs, whose results are all computed again: each chain ends at its first NaN (5 times the
+    time of a finite product; 150 times with chains that run to their end)."""
+    import torch
+    M, N, K = 1024, 8192, 384
+    a, b, c = (torch.randn(*s, device="cuda") for s in ((M, K), (N, K), (M, N)))
+    times = []
+    for value in (None, float("nan")):
+        if value is not None:
+            a.fill_(value)
+        for _ in range(3):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            g.call("nnb200_gemm_f32", g.ptr(a), g.ptr(b), g.ptr(c), M, N, K, K, K, N, 0, 0, C.c_float(1.0), None, None, 0, g.stream())
+            e1.record()
+            torch.cuda.synchronize()
+        times.append(e0.elapsed_time(e1))
+    assert times[1] < 15 * times[0], times
