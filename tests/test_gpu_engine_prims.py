@@ -56,12 +56,18 @@ def test_attention_primitives_match_reference_golden(g):
 
 
 @pytest.mark.parametrize("batch,M,N,K,D,masked", [(4, 64, 64, 32, 32, True), (2, 150, 150, 64, 64, True), (3, 40, 70, 16, 16, False),
-                                                  (1, 130, 257, 8, 8, False)])
+                                                  (1, 130, 257, 8, 8, False),
+                                                  # more than one chunk of 64 in K, more than one walk over the columns of V, K or Q
+                                                  (2, 70, 130, 128, 128, True), (1, 65, 65, 100, 100, False), (2, 40, 70, 136, 200, True),
+                                                  (1, 70, 130, 200, 260, False), (2, 130, 70, 65, 129, True)])
 def test_attention_primitives_match_oracle(g, batch, M, N, K, D, masked):
     r = np.random.default_rng(batch * 1000 + M)
     f = lambda *s: r.standard_normal(s).astype(np.float32)
     A, B, V, G, P = f(batch * K, M), f(batch * K, N), f(batch * N, D), f(batch * M, D), f(batch * M, N)
     mask = np.where(np.arange(N)[None, :] <= np.arange(M)[:, None], 0.0, -np.inf).astype(np.float32) if masked else None
+    if masked and K > 64:                        # the other triangle, and keys at the end for all: the first tile of a walk is closed
+        mask = np.ascontiguousarray(mask[::-1, ::-1])
+        mask[:, -3:] = 0.0
     alpha = 1.0 / np.sqrt(K)
     m, l, O, gq, R, gk, gv = attention_chain(g, A, B, V, G, P, mask, batch, M, N, K, D, float(alpha))
     wm = go.bmm_reduce_max(A, B, batch, alpha, mask)
