@@ -9,8 +9,10 @@
 // The tensor core adds into its accumulator without rounding to nearest, which would drift over a long K: a TMEM
 // accumulator therefore holds one block of 64 k only (small products first) and eight warps add it to fp32 registers,
 // rounding to nearest, while the other TMEM buffer fills.
-// An operand that is not finite, or rounds to infinity in bf16, makes every result it enters NaN or infinite; such a
-// result is computed again with fp32 FMAs (sgemm_exact), which is what the result then is.
+// bf16 has the exponents of fp32, so the lower planes of a small operand (below 2^-110) would fall under its smallest number:
+// what the first plane leaves is enlarged by 2^15 before the other two are taken, and the MMAs take the factor out again.
+// A sum that is not finite (an operand that is not, or beyond 2^121, or a sum beyond 2^115) is computed again with fp32 FMAs
+// (sgemm_exact), which is what the result then is.
 //
 // One CTA per SM, persistent over output tiles of 128 x BN.  All 16 warps do the same work on a quarter of everything: load
 // fp32 from global memory into registers a block of 64 k ahead (any row stride or alignment, either operand contiguous
@@ -35,6 +37,7 @@ namespace {
 
 constexpr int FM = 128, FK = 64, F_THREADS = 512;
 constexpr int F_PLANE_A = FM * FK * 2;                           // one bf16 plane of an A tile, bytes
+constexpr int F_SHIFT = 15;                                      // the residual behind the first plane is enlarged by 2^15
 
 struct F32GemmParams {
     const float* A;
@@ -128,13 +131,18 @@ struct Frag {
                 float x[8];
                 memcpy(x, &v[i][0], 16);
                 memcpy(x + 4, &v[i][1], 16);
+                uint64_t y[4];                                    // pairs: one instruction for two values
+#pragma unroll
+                for (int j = 0; j < 4; ++j) y[j] = pack2(x[2 * j], x[2 * j + 1]);
 #pragma unroll
                 for (int pl = 0; pl < 3; ++pl) {
                     uint32_t h[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
+                        unpack2(y[j], x[2 * j], x[2 * j + 1]);
                         h[j] = pack_bf16x2(x[2 * j], x[2 * j + 1]);
-                        if (pl < 2) { x[2 * j] -= __uint_as_float(h[j] << 16); x[2 * j + 1] -= __uint_as_float(h[j] & 0xffff0000u); }
+                        if (pl < 2) y[j] = fma2(pack2(__uint_as_float(h[j] << 16), __uint_as_float(h[j] & 0xffff0000u)), pack2(-1.f, -1.f), y[j]);
+                        if (pl == 0) y[j] = mul2(y[j], pack2(1 << F_SHIFT, 1 << F_SHIFT));
                     }
                     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + pl * plane), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
                 }
@@ -263,9 +271,10 @@ __global__ void __launch_bounds__(F_THREADS, 1) f32_gemm_kernel(const __grid_con
                 mbar_wait(full0 + 8 * s, (it / STAGES) & 1, abort_flag, 3, &g_f32gemm_error)) {
                 tc_fence_after();
                 const uint32_t a0 = ta, b0 = a0 + 3 * F_PLANE_A, d = tmem_base + a * BN;
-                // plane pairs, the smallest products first
+                // plane pairs, the smallest products first.  The second and third planes are 2^15 too large, so mid * mid is by
+                // 2^30, the others but hi * hi by 2^15: the accumulator is taken down twice by 2^15 on the way
                 constexpr int PAIRS = NB == 3 ? 6 : 3;
-                constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0}, QA[3] = {2, 1, 0};
+                constexpr int PA[6] = {1, 2, 0, 1, 0, 0}, PB[6] = {1, 0, 2, 0, 1, 0}, QA[3] = {2, 1, 0};
 #pragma unroll
                 for (int w = 0; w < PAIRS; ++w) {
                     const uint32_t ap = a0 + (NB == 3 ? PA[w] : QA[w % 3]) * F_PLANE_A, bp = b0 + (NB == 3 ? PB[w] : 0) * PLANE_B;
@@ -273,7 +282,9 @@ __global__ void __launch_bounds__(F_THREADS, 1) f32_gemm_kernel(const __grid_con
                     for (int k = 0; k < FK / 16; ++k) {
                         const uint64_t da = A_MN ? smem_desc(ap + k * (16 * 128), FK * 128, 1024) : smem_desc(ap + k * 32, 16, 1024);
                         const uint64_t db = B_MN ? smem_desc(bp + k * (16 * 128), FK * 128, 1024) : smem_desc(bp + k * 32, 16, 1024);
-                        umma_bf16(d, da, db, IDESC, (w > 0 || k > 0) ? 1u : 0u);
+                        const bool larger = NB == 3 ? w == 1 || w == 5 : w == 2;
+                        if (k == 0 && larger) umma_bf16_shift<F_SHIFT>(d, da, db, IDESC);
+                        else umma_bf16(d, da, db, IDESC, (w > 0 || k > 0) ? 1u : 0u);
                     }
                 }
                 umma_commit(empty0 + 8 * s);

@@ -215,3 +215,20 @@ def test_gemm_f32_full_of_nans_is_not_slow(g):
             torch.cuda.synchronize()
         times.append(e0.elapsed_time(e1))
     assert times[1] < 15 * times[0], times
+
+
+@pytest.mark.parametrize("M,N,K", [(130, 70, 65), (384, 128, 1024), (3000, 2600, 70)])
+@pytest.mark.parametrize("ea,eb", [(-112, 100), (-118, 118), (-126, 120), (-140, 124), (100, -126), (-60, -60), (-120, 0), (40, 40)])
+def test_gemm_f32_keeps_the_bits_of_small_operands(g, M, N, K, ea, eb):
+    """Operands whose lower bits lie below the smallest bf16 number count in full, as they do in fp32 arithmetic."""
+    r = np.random.default_rng(K)
+    A = (r.standard_normal((M, K)) * 2.0 ** ea).astype(np.float32)         # subnormal ones hold the bits that fp32 has for them
+    B = (r.standard_normal((N, K)) * 2.0 ** eb).astype(np.float32)
+    a, b, c = g.dev(A), g.dev(B), g.dev(np.zeros((M, N), np.float32))
+    g.call("nnb200_gemm_f32", g.ptr(a), g.ptr(b), g.ptr(c), M, N, K, K, K, N, 0, 0, C.c_float(1.0), None, None, 0, g.stream())
+    want = A.astype(np.float64) @ B.astype(np.float64).T
+    scale = np.abs(A.astype(np.float64)) @ np.abs(B.astype(np.float64)).T
+    # the bound of test_gemm_f32_against_float64, and half the smallest fp32 number for results down there
+    bound = scale * (2.0 ** -24 + 6 * 2.0 ** -23 + (K / 64 + 8) * 2.0 ** -24) + 2.0 ** -23 * np.abs(want) + 2.0 ** -149
+    assert (np.abs(g.host(c) - want) <= bound).all()
+    assert g.gemm_status() == 0
