@@ -7,7 +7,7 @@
 // products replace one fp32 FMA, at 1/6 of the bf16 rate against 1/32 of it on the fp32 pipe.  With a bf16 operand B
 // (weights of the decoding path) three products are exact.
 // The tensor core adds into its accumulator without rounding to nearest, which would drift over a long K: a TMEM
-// accumulator therefore holds one block of 64 k only (small products first) and eight warps add it to fp32 registers,
+// accumulator therefore holds one block of 64 k only (small products first) and all warps add it to fp32 registers,
 // rounding to nearest, while the other TMEM buffer fills.
 // bf16 has the exponents of fp32, so the lower planes of a small operand (below 2^-110) would fall under its smallest number:
 // what the first plane leaves is enlarged by 2^15 before the other two are taken, and the MMAs take the factor out again.
@@ -238,7 +238,8 @@ __global__ void __launch_bounds__(F_THREADS, 1) f32_gemm_kernel(const __grid_con
     const uint32_t my_tmem = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + colw;
 
     // A wait that gives up sets the abort flag, after which every other wait returns at once: the loops run to their end
-    // with the same barriers on all warps, and nothing is written.
+    // with the same barriers on all warps, and this CTA writes nothing.  What it hands to the peers of a cluster is NaN, so that
+    // they compute their results again instead of adding up an unfinished tile.
     int it = 0;
     for (int u = first; u < units; u += step) {
         float acc[HC];
@@ -298,6 +299,10 @@ __global__ void __launch_bounds__(F_THREADS, 1) f32_gemm_kernel(const __grid_con
         // every MMA has been waited for, so the operand stages are free for the sums on their way out
         if (CLUSTER) {
             float* part = reinterpret_cast<float*>(smem) + (q * 32 + lane) * (BN + 4) + colw;
+            if (*abort_flag) {
+#pragma unroll
+                for (int j = 0; j < HC; ++j) acc[j] = __int_as_float(0x7fc00000);
+            }
 #pragma unroll
             for (int j = 0; j < HC; j += 4) *reinterpret_cast<float4*>(part + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
         } else {
