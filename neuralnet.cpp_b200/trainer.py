@@ -347,7 +347,8 @@ class GptTrainer:
         n = len(tokens)
         if not (n >= 1 and 0 <= int(cur_len) and int(cur_len) + n <= self.cfg.seq):
             raise ValueError("the rows [cur_len, cur_len + tokens) must lie in [0, seq)")
-        ids = np.ascontiguousarray(tokens, np.int32)
+        # 32 bits of each id, as forward_step passes them: ids out of the vocabulary's range are zero rows, however large
+        ids = np.array([int(t) & 0xffffffff for t in tokens], np.uint32).view(np.int32)
         self._capture_step(ids[0], cur_len, cur_len)         # not in the first token behind the prompt; row cur_len is written again below
         call("nnb200_gpt_prefill", C.byref(self._c), _ptr(self.params), _ptr(self.shadow), _ptr(ws), C.c_void_p(ids.ctypes.data), n,
              int(cur_len), _ptr(logits), _stream())

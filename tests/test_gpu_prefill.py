@@ -71,3 +71,16 @@ def test_prompt_in_page_locked_memory_may_be_overwritten_after_the_call(n):
     buf.fill_(1)
     torch.cuda.synchronize()
     assert torch.equal(logits, want)
+
+
+def test_ids_beyond_32_bits_are_what_single_steps_make_of_them():
+    """A prompt of ids no 32-bit integer holds, which steps take as zero rows (or modulo 2^32), and of 0-d tensors."""
+    import torch
+    from tests.gpu_util import nnb
+    tr = _trainer(nnb, 72, 32, 1, 1, 64, 16, 1, 1, 2, 0)
+    tokens = [3, 2 ** 31 + 5, 7, 2 ** 32 + 9, -1, 70, 2 ** 40, 1, torch.tensor(5), 6]
+    for i, t in enumerate(tokens):
+        want = tr.forward_step(int(t), i, i)
+    want = want.clone()
+    assert rel_err(tr.prefill(tokens).cpu().numpy(), want.cpu().numpy()) < 1e-5
+    assert len(tr.generate(tokens[:8] + [int(tokens[8])], 2, temperature=0.0)) == 2
