@@ -25,6 +25,7 @@ ACT_GELU, ACT_SWIGLU = 0, 1
 NORM_LAYER, NORM_RMS = 0, 1
 POS_LEARNED, POS_SINUSOIDAL, POS_ALIBI, POS_ROPE = 0, 1, 2, 3
 FP32, BF16 = 0, 1
+PROMPT_MIN = 8       # kPromptMin of csrc/decode.cu: prompts from here on go through the model at once
 
 
 @dataclasses.dataclass
@@ -367,7 +368,7 @@ class GptTrainer:
 
         def fill(start):
             nonlocal cur_len, last
-            if len(context) - start >= 8:            # shorter ones are quicker a token at a time
+            if len(context) - start >= PROMPT_MIN:   # shorter ones are quicker a token at a time
                 last = self.prefill(context[start:], cur_len)
                 cur_len += len(context) - start
                 return

@@ -29,3 +29,8 @@ def test_dependent_kernels_do_not_promise_constant_memory():
         early = body[:body.index("pdl_wait()")]
         for produced in re.findall(r"const float\* (\w+)", params):
             assert not re.search(rf"(?<!<uintptr_t>\()\b{produced}\s*(\[|\+)", early), (name, produced)
+
+
+def test_the_shortest_prompt_of_a_pass_is_the_same_for_host_and_library():
+    import __graft_entry__ as entry
+    assert int(re.search(r"constexpr int kPromptMin = (\d+);", open(SOURCE).read()).group(1)) == entry.load_package().trainer.PROMPT_MIN
