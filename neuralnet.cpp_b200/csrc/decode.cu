@@ -32,7 +32,8 @@ struct DecodeWs { size_t kv, table, x, qkv, att, xmid, h2, logits, step, total;
 // Rows of a prompt that one pass takes (longer prompts go in several): enough to fill the GEMM's tiles, 60 MB of
 // activations for a model of width 1024.
 constexpr int kPromptRows = 1024;
-// Shorter prompts go through the single-token kernels: a pass costs about as much as several tokens whatever its length.
+// Shorter prompts go through the single-token kernels: a pass costs as much as four to six tokens whatever its length (us for 4 and 6
+// tokens as steps | a pass: 2 layers of 128: 126, 187 | 120; 6 of 384: 320, 476 | 450; 12 of 768: 873, 1304 | 1100).
 constexpr int kPromptMin = 8;
 static DecodeWs decode_ws(const nnb200_gpt_config& c)
 {
@@ -132,8 +133,8 @@ __global__ void decode_embed_kernel(const float* __restrict__ tok_emb, const flo
 //   NORM: f = norm(x) * gamma (+ beta), eps 1e-5 inside the rsqrt (compute_layer.hpp:495, 687; LayerNorm when `layer`).
 //   ACT 1: SwiGLU, y[o] = gate * sigmoid(gate) * up of rows o and o + out (compute_layer.hpp:375-404), R = 2;
 //   ACT 2: QuickGeLU (:266-295).
-// R is 1 where there are too few rows for more than a warp each (latency), 4 for the LM head (12 us of bytes: fewer
-// stagings of x per row).
+// R is 1 where there are too few rows for more than a warp each (latency), 4 for the LM head (8192 rows and more: fewer blocks
+// that each stage x).
 template <typename WT, bool NORM, int R, int ACT>
 __global__ void __launch_bounds__(256, 3) gemv_kernel(const WT* __restrict__ W, const float* x, const float* __restrict__ gamma,
                                                    const float* __restrict__ beta, int layer, const float* __restrict__ bias,

@@ -17,9 +17,11 @@ namespace nnb {
 
 // The five attention primitives work on 64 x 64 tiles of the scores (simt_tile.cuh); a block owns a tile row (or column,
 // for the key / value gradients) of one batch entry and walks the tiles of the other index, leaving out tiles whose mask is
-// -inf throughout (half of them under a causal mask).  They are bound by the fp32 pipe: the score product is done again in
-// every primitive, because each is a call of its own that gets no scores.  At 48 x 256 x 256 x 64 (causal) the chain of six
-// calls takes 308 us, and took 2360 us with one warp per row and a dot product per score.
+// -inf throughout (half of them under a causal mask).  The score product is done again in every
+// primitive, because each is a call of its own that gets no scores.  At 48 x 256 x 256 x 64 (causal) the chain of six calls takes
+// 333 us, and took 2572 us with one warp per row and a dot product per score.  What bounds it is latency: staging by scalar
+// loads, two barriers and a product with no load in flight per tile, and 192 blocks of unequal length on 148 SMs; the 2.5 GFLOP
+// are about 8 of the fp32 pipe's 70 TFLOP/s.
 struct BmmDims {
     int batch, M, N, K, transA, transB;
     float alpha;
